@@ -6,13 +6,16 @@
 //   E = clip(clip(H^p, void, 1) * E_mul, void, inf),   dE = p H^(p-1) H'(r) E_mul.
 //
 // OC (pyFANTOM/Optimizers/CUDA/OC.py:67-129) bisects the Lagrange multiplier with the host
-// testing g(x_new) after every step.  Here a pass evaluates the constraint at all 31
-// midpoints of the next five levels of the bisection tree in one sweep over the elements
-// (one partial sum per midpoint and block), and a one-block kernel replays the five
-// sequential decisions with the reference's stopping rule; the midpoints are formed
-// exactly as the sequential loop forms them, so the sequence of (l1, l2) is the same.
+// testing g(x_new) after every step.  Here a pass evaluates the constraint at many midpoints
+// in one sweep over the elements (one partial sum per midpoint and block); its last block
+// adds the partial sums and replays the sequential decisions with the reference's stopping
+// rule; the midpoints are formed exactly as the sequential loop forms them, so the sequence
+// of (l1, l2) is the same.  See k_oc_pass for the single constraint; with several constraints
+// (k_oc_eval, k_oc_step_multi) each pass covers the 31 midpoints of five bisection levels.
 #include <cmath>
+#include <cstddef>
 
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -163,24 +166,6 @@ __device__ void oc_tree(OcState* S) {
     }
 }
 
-__global__ void __launch_bounds__(kRT) k_oc_init(const double* partials, int np, OcState* S) {
-    __shared__ double s_red[kRT / 32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) s += partials[i];
-    s = block_sum<kRT>(s, s_red);
-    if (threadIdx.x == 0) {
-        S->abs_sum = s;
-        S->allzero = s == 0.0;
-        S->l1 = 1e-9;
-        S->l2 = 1e9;
-        S->lmid = 0.0;
-        S->done = 0;
-        S->steps = 0;
-        S->change2 = 0.0;
-        oc_tree(S);
-    }
-}
-
 __device__ __forceinline__ double oc_xnew(double xi, double oc, double lam, double move) {
     const double xu = fmin(fmax(xi + move, 0.0), 1.0), xl = fmin(fmax(xi - move, 0.0), 1.0);
     return fmax(0.0, fmax(xl, fmin(1.0, fmin(xu, oc / lam))));
@@ -217,44 +202,6 @@ __global__ void __launch_bounds__(kRT) k_oc_eval(long long n, const double* __re
     }
 }
 
-__global__ void __launch_bounds__(32) k_oc_step(const double* partials, int np, double vf, OcState* S) {
-    if (S->done) return;
-    const int t = threadIdx.x;
-    if (t < kOcTree) {
-        double s = 0.0;
-        for (int b = 0; b < np; b++) s += partials[(long long)b * kOcTree + t];
-        S->g[t] = s - vf;
-    }
-    __syncwarp();
-    if (t == 0) {
-        int node = 0;
-        for (int d = 0; d < 5; d++) {
-            const double l1 = S->l1, l2 = S->l2;
-            if (!((l2 - l1) / (l2 + l1) > 1e-8)) {
-                S->done = 1;
-                break;
-            }
-            const double lmid = S->lam[node];
-            S->lmid = lmid;
-            S->steps += 1;
-            if (S->g[node] <= 0.0) {
-                S->l2 = lmid;
-                node = 2 * node + 1;
-            } else {
-                S->l1 = lmid;
-                node = 2 * node + 2;
-            }
-        }
-        if (!S->done) {
-            const double l1 = S->l1, l2 = S->l2;
-            if (!((l2 - l1) / (l2 + l1) > 1e-8))
-                S->done = 1;
-            else
-                oc_tree(S);
-        }
-    }
-}
-
 __global__ void __launch_bounds__(kRT) k_oc_write(long long n, const double* __restrict__ x, const double* __restrict__ ocp,
                                                   double move, const OcState* S, double* __restrict__ xnew,
                                                   double* partials) {
@@ -270,14 +217,6 @@ __global__ void __launch_bounds__(kRT) k_oc_write(long long n, const double* __r
     }
     s = block_sum<kRT>(s, s_red);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
-}
-
-__global__ void __launch_bounds__(kRT) k_oc_change(const double* partials, int np, OcState* S) {
-    __shared__ double s_red[kRT / 32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < np; i += blockDim.x) s += partials[i];
-    s = block_sum<kRT>(s, s_red);
-    if (threadIdx.x == 0) S->change2 = s;
 }
 
 // Several volume constraints (one per material, variables material-major): the reference
@@ -355,6 +294,345 @@ __global__ void __launch_bounds__(kRT) k_oc_init_multi(const double* partials, i
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// OC with one constraint
+// ---------------------------------------------------------------------------------------
+// The sequential loop starts with the bracket [1e-9, 1e9]; as long as g(mid) <= 0 the next
+// midpoint is (1e-9 + mid) / 2.  These midpoints (the spine) are known in advance.  For
+// dg >= 0 the volume g falls with the multiplier, so the first spine point with g > 0 is found
+// in two passes: every 11th spine point (fused with the computation of ocP), then the ten
+// between two of them.  The bracket then spans a factor of two, and each further pass covers
+// the 15 midpoints of four bisection levels (31 of five need more registers than two blocks
+// per SM leave): 9 passes in all.  Within a pass an element whose x_new sits on the same
+// bound (or on neither) for the whole bracket adds one term instead of 15; after the first
+// pass or two of the tree almost every element does.  Where dg is not a finite number >= 0,
+// or ocP vanishes everywhere (x_new = 1e-3 / lambda), every pass covers four levels from the
+// start: more passes, the same sequence.
+// Bound by the FP64 pipe in the first three passes (a product, two comparisons and an FMA
+// per element and midpoint; the reciprocal of the midpoint replaces the division in these
+// sums, x_new itself is divided) and by reading x, ocP and dg (24 B per element, from L2 up
+// to about 4 M elements) in the others.
+constexpr int kOcStride = 11;
+constexpr int kOcMid = 15;  // midpoints of four bisection levels
+
+
+struct OcSpine {
+    int n;
+    double m[96];
+};
+
+struct OcRun {
+    double change2, lmid;
+    int steps, done;
+    double l1, l2, blo, bhi;  // bracket; smallest and largest midpoint of the pass
+    int mode;                 // 0 four levels of the tree, 1 coarse spine, 2 fine spine
+    int ne, base, hipos;      // midpoints of the pass; fine spine: its first index, g > 0 behind it
+    int allzero, flags;       // flags: 1 some dg not finite >= 0, 2 some ocP != 0
+    int listed;               // 1: the warps hold lists of the elements still undecided
+    unsigned count;           // blocks of the running pass that have finished
+    double lam[kOcMid];
+};
+static_assert(sizeof(OcRun) <= sizeof(OcState), "OcRun shares the workspace of OcState");
+
+// one element's terms of the constraint at NE midpoints; true if they differ by more than a
+// common constant (cst) or a common constant over the multiplier (lin)
+template <int NE>
+__device__ __forceinline__ bool oc_accumulate(double xi, double oc, double d, double move, const double* s_r, double rlo,
+                                              double rhi, double& cst, double& lin, double (&acc)[kOcMid]) {
+    const double xu = fmin(fmax(xi + move, 0.0), 1.0), xl = fmin(fmax(xi - move, 0.0), 1.0);
+    const double vmax = oc * rlo, vmin = oc * rhi;  // oc over the smallest and largest midpoint
+    const bool up = vmin >= xu, low = vmax <= xl, mid = vmin >= xl && vmax <= xu;
+    if (up || low) {
+        cst += d * (up ? xu : xl);
+        return false;
+    }
+    if (mid) {
+        lin += d * oc;
+        return false;
+    }
+#pragma unroll
+    for (int t = 0; t < NE; t++) {
+        double v = oc * s_r[t];
+        v = v < xu ? v : xu;  // as fmin and fmax, a NaN gives the bound
+        v = v > xl ? v : xl;
+        acc[t] += d * v;
+    }
+    return true;
+}
+
+// decisions after a pass (one block; g[0..ne) in shared memory); writes the next midpoints
+__device__ void oc_decide(OcRun* S, const OcSpine& sp, const double* g, int mode, int ne, int base, int hipos, int flags,
+                          const double* s_lam) {
+    __shared__ int s_next;  // next mode, -1: done
+    if (threadIdx.x == 0) {
+        int next = 0;
+        if (mode == 1) {
+            S->allzero = !(flags & 2);
+            if ((flags & 1) || !(flags & 2)) {
+                S->l1 = 1e-9, S->l2 = 1e9, S->lmid = 0.0, S->steps = 0;
+            } else {
+                int j = 0;
+                while (j < ne && g[j] <= 0.0) j++;
+                S->base = j * kOcStride;
+                S->hipos = j < ne;
+                S->ne = j < ne ? kOcStride - 1 : sp.n - j * kOcStride;
+                next = 2;
+            }
+        } else if (mode == 2) {
+            int q = 0;
+            while (q < ne && g[q] <= 0.0) q++;
+            if (q == ne && !hipos) {  // g <= 0 down to the end of the bisection
+                S->l1 = 1e-9, S->l2 = S->lmid = sp.m[sp.n - 1], S->steps = sp.n;
+            } else {
+                const int k = base + q;
+                S->l1 = S->lmid = sp.m[k];
+                S->l2 = k > 0 ? sp.m[k - 1] : 1e9;
+                S->steps = k + 1;
+            }
+        } else {
+            int node = 0;
+            double l1 = S->l1, l2 = S->l2, lmid = S->lmid;
+            int steps = S->steps;
+            for (int d = 0; d < 4; d++) {
+                if (!((l2 - l1) / (l2 + l1) > 1e-8)) break;
+                lmid = s_lam[node];
+                steps++;
+                if (g[node] <= 0.0) {
+                    l2 = lmid;
+                    node = 2 * node + 1;
+                } else {
+                    l1 = lmid;
+                    node = 2 * node + 2;
+                }
+            }
+            S->l1 = l1, S->l2 = l2, S->lmid = lmid, S->steps = steps;
+        }
+        if (next == 0) {
+            const double l1 = S->l1, l2 = S->l2;
+            S->done = !((l2 - l1) / (l2 + l1) > 1e-8);
+            S->ne = kOcMid;
+            S->blo = l1, S->bhi = l2;
+        } else {
+            S->blo = sp.m[S->base + S->ne - 1 + (S->ne == 0)], S->bhi = sp.m[S->base];
+        }
+        S->mode = next;
+        S->count = 0;
+        s_next = next;
+    }
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t >= kOcMid) return;
+    if (s_next == 2) {
+        if (t < S->ne) S->lam[t] = sp.m[S->base + t];
+        return;
+    }
+    // heap layout: node t covers (a, b), its midpoint is (a + b) / 2; the left child (a, mid)
+    // follows g(mid) <= 0 (l2 = mid), the right child (mid, b) otherwise
+    double a = S->l1, b = S->l2, m = (a + b) / 2.0;
+    const int depth = 31 - __clz(t + 1);
+    for (int d = depth - 1; d >= 0; d--) {
+        if (((t + 1) >> d) & 1)
+            a = m;
+        else
+            b = m;
+        m = (a + b) / 2.0;
+    }
+    S->lam[t] = m;
+}
+
+// ints of x_new for each warp's list (even: the list starts with two sums)
+__host__ __device__ inline int oc_list_room(long long n, unsigned nb) { return (int)(2 * n / ((long long)nb * (kRT / 32))) & ~1; }
+
+// KIND 0: the first pass; 1: any later pass over all elements; 2: a pass over the warps' lists
+// (does nothing before they are built), a kernel of its own so that its few instructions are
+// not fetched between the unrolled sweeps of the others
+template <int KIND>
+__global__ void __launch_bounds__(kRT, 2) k_oc_pass(long long n, const double* __restrict__ x, const double* __restrict__ df,
+                                                 const double* __restrict__ dg, double* __restrict__ ocp, double move,
+                                                 double vf, const __grid_constant__ OcSpine sp, OcRun* S,
+                                                 double* partials, int* lists) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr bool FIRST = KIND == 0;
+    constexpr int NWp = kRT / 32;
+    __shared__ double s_lam[kOcMid], s_r[kOcMid], s_g[kOcMid];
+    __shared__ double s_part[NWp][kOcMid + 2];
+    __shared__ int s_last;
+    const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    // the state in one round of loads
+    const int done = FIRST ? 0 : S->done, mode = FIRST ? 1 : S->mode, ne = FIRST ? sp.n / kOcStride : S->ne;
+    const int base = FIRST ? 0 : S->base, hipos = FIRST ? 0 : S->hipos, inlist = FIRST ? 0 : S->listed;
+    const double lam = FIRST ? (tid < ne ? sp.m[kOcStride * tid + kOcStride - 1] : 1.0) : S->lam[tid < kOcMid ? tid : 0];
+    const double blo0 = FIRST ? 1.0 : S->blo, bhi0 = FIRST ? 1.0 : S->bhi;
+    const bool allzero = FIRST ? false : S->allzero != 0;
+    if (done || (KIND == 2 && !inlist)) return;
+    if (tid < ne) {
+        const double v = lam;
+        s_lam[tid] = v;
+        s_r[tid] = 1.0 / v;
+    } else if (tid < kOcMid) {
+        s_lam[tid] = 1.0;
+        s_r[tid] = 1.0;
+    }
+    __syncthreads();
+    const double blo = FIRST ? s_lam[ne - 1] : blo0, bhi = FIRST ? s_lam[0] : bhi0;
+    const double rlo = 1.0 / blo, rhi = 1.0 / bhi;
+    double acc[kOcMid], cst = 0.0, lin = 0.0;
+#pragma unroll
+    for (int t = 0; t < kOcMid; t++) acc[t] = 0.0;
+    int flags = 0;
+    // warp-uniform loop over runs of 32 elements, several of them loaded ahead of their use
+    const long long wstep = (long long)gridDim.x * kRT, w0 = (long long)blockIdx.x * kRT + w * 32;
+    int listed = 0;  // entries of this warp's list of undecided elements
+    const int lcap = oc_list_room(n, gridDim.x);
+    int* seg = lists ? lists + ((long long)blockIdx.x * NWp + w) * lcap : nullptr;
+    auto sweep = [&](auto NEc, bool build) {
+        constexpr int NE = decltype(NEc)::value, kOcBatch = 4;
+        for (long long k0 = w0; k0 < n; k0 += kOcBatch * wstep) {
+            double xv[kOcBatch], ov[kOcBatch], dv[kOcBatch];
+#pragma unroll
+            for (int q = 0; q < kOcBatch; q++) {
+                const long long i = k0 + q * wstep + l;
+                const bool ok = i < n;
+                xv[q] = ok ? x[i] : 0.0;
+                dv[q] = ok ? dg[i] : 0.0;
+                ov[q] = ok ? (FIRST ? df[i] : ocp[i]) : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < kOcBatch; q++) {
+                const long long i = k0 + q * wstep + l;
+                const bool ok = i < n;
+                double oc = ov[q];
+                if constexpr (FIRST) {
+                    double r = sqrt(fmax(-oc / dv[q], 0.0));
+                    if (r != r) r = 0.0;
+                    oc = ok ? xv[q] * r : 0.0;
+                    if (ok) ocp[i] = oc;
+                    if (!(dv[q] >= 0.0) || isinf(dv[q])) flags |= 1;
+                    if (oc != 0.0) flags |= 2;
+                } else if (allzero && ok) {
+                    oc = 1e-3;
+                }
+                const bool act = oc_accumulate<NE>(xv[q], oc, dv[q], move, s_r, rlo, rhi, cst, lin, acc);
+                if (build) {
+                    const unsigned m = __ballot_sync(0xffffffffu, act);
+                    if (act) seg[6 + listed + __popc(m & ((1u << l) - 1u))] = (int)i;
+                    listed += __popc(m);
+                }
+            }
+        }
+    };
+    const bool build = KIND == 1 && lists && mode == 0 && !inlist && bhi < 1.5 * blo;
+    if constexpr (FIRST) {
+        sweep(std::integral_constant<int, kOcStride - 1>{}, false);
+    } else if constexpr (KIND == 2) {
+        // the sums of the elements decided for the bracket of the building pass, then the others
+        double* head = reinterpret_cast<double*>(seg);
+        const int cnt = seg[4];
+        if (l == 0) cst = head[0], lin = head[1];
+        for (int q = l; q < cnt; q += 32) {
+            const int i = seg[6 + q];
+            oc_accumulate<kOcMid>(x[i], allzero ? 1e-3 : ocp[i], dg[i], move, s_r, rlo, rhi, cst, lin, acc);
+        }
+    } else if (mode == 2) {
+        sweep(std::integral_constant<int, kOcStride - 1>{}, false);
+    } else {
+        sweep(std::integral_constant<int, kOcMid>{}, build);
+    }
+    cst = warp_sum(cst);
+    lin = warp_sum(lin);
+    if (l == 0) s_part[w][kOcMid] = cst, s_part[w][kOcMid + 1] = lin;
+    if (build && l == 0) {
+        double* head = reinterpret_cast<double*>(seg);
+        head[0] = cst, head[1] = lin;
+        seg[4] = listed;
+    }
+#pragma unroll
+    for (int t = 0; t < kOcMid; t++) {
+        if (t < ne) {  // uniform over the grid
+            const double v = warp_sum(acc[t]);
+            if (l == 0) s_part[w][t] = v;
+        }
+    }
+    if (FIRST) flags = __reduce_or_sync(0xffffffffu, flags);
+    if (FIRST && l == 0 && flags) atomicOr(&S->flags, flags);
+    __syncthreads();
+    if (tid < ne) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < NWp; k++) s += s_part[k][tid] + s_part[k][kOcMid] + s_part[k][kOcMid + 1] * s_r[tid];
+        partials[(long long)blockIdx.x * kOcMid + tid] = s;
+    }
+    // the last block to get here adds the partial sums (in block order) and decides
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&S->count, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    {  // thread (t, group): every 16th block's sum for midpoint t
+        const int t = tid & 15;
+        double s = 0.0;
+        if (t < ne) {
+#pragma unroll 4
+            for (unsigned b = tid >> 4; b < gridDim.x; b += kRT / 16) s += __ldcg(partials + (long long)b * kOcMid + t);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+        if (l < 16) s_part[w][t] = s;  // 17 columns a row
+    }
+    __syncthreads();
+    if (tid < ne) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < NWp; k++) s += s_part[k][tid];
+        s_g[tid] = s - vf;
+    }
+    __syncthreads();
+    if (build && tid == 0) S->listed = 1;
+    oc_decide(S, sp, s_g, mode, ne, base, hipos, FIRST ? *(volatile int*)&S->flags : 0, s_lam);
+}
+
+// x_new and ||x_new - x||^2 (partial sums, added by the last block); without `force` only once
+// the bisection has ended
+__global__ void __launch_bounds__(kRT) k_oc_final(long long n, const double* x, const double* __restrict__ ocp, double move,
+                                                  OcRun* S, int force, double* xnew, double* partials) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double s_red[kRT / 32];
+    __shared__ int s_last;
+    if (!force && !S->done) return;
+    const double lam = S->lmid;
+    const bool allzero = S->allzero != 0;
+    double s = 0.0;
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * kRT + threadIdx.x; i < n; i += (long long)gridDim.x * kRT) {
+        const double xi = x[i], v = oc_xnew(xi, allzero ? 1e-3 : ocp[i], lam, move);
+        xnew[i] = v;
+        s += (xi - v) * (xi - v);
+    }
+    s = block_sum<kRT>(s, s_red);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = s;
+        __threadfence();
+        s_last = atomicAdd(&S->count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    s = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += kRT) s += __ldcg(partials + b);
+    s = block_sum<kRT>(s, s_red);
+    if (threadIdx.x == 0) S->change2 = s, S->count = 0;
+}
+
+static OcSpine oc_spine() {
+    OcSpine sp;
+    sp.n = 0;
+    const double l1 = 1e-9;
+    for (double l2 = 1e9; (l2 - l1) / (l2 + l1) > 1e-8; l2 = sp.m[sp.n++]) sp.m[sp.n] = (l1 + l2) / 2.0;
+    return sp;
+}
+
 static unsigned oc_blocks(long long n) {
     long long nb = (n + kRT - 1) / kRT;
     if (nb > 2LL * kNumSM) nb = 2LL * kNumSM;
@@ -370,26 +648,44 @@ int oc_update(long long n, const double* x, const double* df, const double* dg, 
     const unsigned nb = oc_blocks(n);
     double* ocp = work;
     double* partials = work + n;
-    OcState* S = reinterpret_cast<OcState*>(partials + (size_t)nb * kOcTree);
-    pf::count_launch();
-    k_oc_prep<<<nb, kRT, 0, st>>>(n, x, df, dg, ocp, partials);
-    pf::count_launch();
-    k_oc_init<<<1, kRT, 0, st>>>(partials, nb, S);
-    for (int p = 0; p < kOcPasses; p++) {
+    OcRun* S = reinterpret_cast<OcRun*>(partials + (size_t)nb * kOcTree);
+    static const OcSpine sp = oc_spine();
+    // until it is written, x_new holds the lists of undecided elements (unless it is x itself,
+    // or too short for each warp's whole share and the list's head)
+    const long long share = 32 * ((n + (long long)nb * kRT - 1) / ((long long)nb * kRT));
+    int* lists = n < (1LL << 31) && x_new != x && share + 6 <= oc_list_room(n, nb) ? reinterpret_cast<int*>(x_new) : nullptr;
+    PF_CUDA(cudaMemsetAsync(S, 0, sizeof(OcRun), st));
+    auto passes = [&](int count, int list_passes) {
+        for (int p = 0; p < count + list_passes; p++) {
+            pf::count_launch();
+            PF_CUDA(launch_pdl(p < count ? k_oc_pass<1> : k_oc_pass<2>, dim3(nb), dim3(kRT), 0, st, n, x, df, dg, ocp, move, vf, sp, S, partials, lists));
+        }
+        return (int)PF_OK;
+    };
+    auto final = [&](int force) {
         pf::count_launch();
-        k_oc_eval<<<nb, kRT, 0, st>>>(n, x, ocp, dg, move, S, partials);
-        pf::count_launch();
-        k_oc_step<<<1, 32, 0, st>>>(partials, nb, vf, S);
-    }
+        PF_CUDA(launch_pdl(k_oc_final, dim3(nb), dim3(kRT), 0, st, n, x, (const double*)ocp, move, S, force, x_new, partials));
+        PF_LAUNCH_CHECK("oc launch");
+        return (int)PF_OK;
+    };
+    int s;
     pf::count_launch();
-    k_oc_write<<<nb, kRT, 0, st>>>(n, x, ocp, move, S, x_new, partials);
-    pf::count_launch();
-    k_oc_change<<<1, kRT, 0, st>>>(partials, nb, S);
-    PF_LAUNCH_CHECK("oc launch");
+    PF_CUDA(launch_pdl(k_oc_pass<0>, dim3(nb), dim3(kRT), 0, st, n, x, df, dg, ocp, move, vf, sp, S, partials, lists));
+    // fine spine, then the 25 levels below a bracket of a factor of two, the first eight of them
+    // over all elements; a caller that does not wait for the result gets the passes of the
+    // general sequence (86 levels) too
+    if ((s = lists ? passes(3, 5) : passes(8, 0)) || (!h_out && (s = passes(kOcPasses - 3, 0)))) return s;
+    if ((s = final(h_out ? 0 : 1))) return s;
     if (h_out) {
-        OcState h;
-        PF_CUDA(cudaMemcpyAsync(&h, S, sizeof(OcState), cudaMemcpyDeviceToHost, st));
+        OcRun h;
+        constexpr size_t head = offsetof(OcRun, l1);  // the results come first
+        PF_CUDA(cudaMemcpyAsync(&h, S, head, cudaMemcpyDeviceToHost, st));
         PF_CUDA(cudaStreamSynchronize(st));
+        if (!h.done) {
+            if ((s = passes(kOcPasses - 3, 0)) || (s = final(1))) return s;
+            PF_CUDA(cudaMemcpyAsync(&h, S, head, cudaMemcpyDeviceToHost, st));
+            PF_CUDA(cudaStreamSynchronize(st));
+        }
         h_out[0] = sqrt(h.change2);
         h_out[1] = h.lmid;
         h_out[2] = (double)h.steps;

@@ -66,3 +66,51 @@ def test_filter_taps_that_are_no_columns(lib):
     lib.check(L.pf_filter_fwd_f64(f, lib.ptr(vt), lib.ptr(y), lib.stream()))
     assert rel(N(y), O.filter_fwd(nel, w, off, v)) < 1e-13
     L.pf_filter_destroy(f)
+
+
+def _oc(lib, x, df, dg, vf, move, wait=True):
+    L = lib.load()
+    n = len(x)
+    xt, ft, gt = T(x), T(df), T(dg)
+    work = torch.full((int(L.pf_oc_workspace_size(n)),), np.nan, dtype=torch.float64, device="cuda")
+    xn = torch.full_like(xt, np.nan)
+    out = (ctypes.c_double * 3)()
+    lib.check(L.pf_oc_update_f64(n, lib.ptr(xt), lib.ptr(ft), lib.ptr(gt), vf, move, lib.ptr(xn), lib.ptr(work),
+                                 out if wait else None, lib.stream()))
+    return N(xn), list(out)
+
+
+@pytest.mark.parametrize("n", [1, 31, 255, 257, 4800, 75_777, 300_001])
+@pytest.mark.parametrize("kind", ["usual", "tiny", "huge", "slack", "tight", "zero", "signs", "flat"])
+def test_oc_sequences(lib, n, kind):
+    # multipliers over the whole bracket, volumes met everywhere or nowhere, a zero gradient,
+    # a constraint gradient of both signs (no falling volume: five levels a pass from the start)
+    rng = np.random.default_rng(n)
+    x = rng.uniform(0.05, 0.95, n)
+    df = -np.exp(rng.normal(0.0, 2.0, n))
+    dg = rng.uniform(0.5, 1.5, n) / n
+    vf, move = 0.4 * dg.sum(), 0.2
+    if kind == "tiny":
+        df = df * 1e-18 / n
+    elif kind == "huge":
+        df = df * 1e14
+    elif kind == "slack":
+        vf = 2.0
+    elif kind == "tight":
+        vf = -1.0
+    elif kind == "zero":
+        df = np.abs(df)
+    elif kind == "signs":
+        dg = np.where(rng.uniform(size=n) < 0.2, -dg, dg)
+    elif kind == "flat":
+        x, df, dg = np.full(n, 0.4), np.full(n, -1.0), np.full(n, 1.0 / n)
+    ref, steps = O.oc_update(x, df, dg, vf, move)
+    got, out = _oc(lib, x, df, dg, vf, move)
+    assert int(out[2]) == steps
+    # the sums differ in order only: the bisection ends within its own tolerance of 1e-8, and
+    # takes another branch only where the volume is met to 1e-13
+    assert np.abs(got - ref).max() < 1e-9 or kind == "flat"
+    if kind == "flat":  # every element at the volume fraction itself: the last steps are ties
+        assert np.abs(got - ref).max() < 2e-8
+    late, _ = _oc(lib, x, df, dg, vf, move, wait=False)
+    assert np.array_equal(late, got)
