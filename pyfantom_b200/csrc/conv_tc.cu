@@ -12,16 +12,20 @@
 //               ones (the bias gradient): A[m, k] = x[n, ci, s*o + t - 1], B[co, k] = dy[n, co, o]
 // Layouts are those of the FP32 kernels (cnn.cu): [N][C][X][Y][Z], weights [Cout][Cin][27].
 //
-// One CTA of 128 threads computes 128 rows (voxels, or weight-gradient rows) against all
-// columns (channels, padded to NP, a multiple of 16).  The reduction runs in chunks of 64:
-// each thread gathers its row's 64 operands (8 x 16 bytes of BF16) into the canonical
-// no-swizzle K-major layout (core matrices of 8 rows x 16 bytes), the threads stage the
-// other operand's slice, and one thread issues four 128 x NP x 16 MMAs and commits them to
-// the buffer's mbarrier.  Two buffers alternate, so the gather of chunk c+1 overlaps the
-// MMAs of chunk c.  After the last chunk each warp reads its 32 rows of the accumulator
-// (tcgen05.ld 32x32b) and stores them column by column (32 consecutive rows per store).
-// Every wait on an mbarrier is bounded: past the limit the kernel records an error in
-// `err`, skips the epilogue, and releases its tensor memory.
+// The im2col matrix is never formed.  A CTA stages the source voxels of its output tile with
+// their halo once per 16 reduction channels, as BF16 in groups of 8 channels (16 bytes per
+// voxel and group, voxels consecutive along z).  In that layout 8 z-neighbours are one core
+// matrix of the tensor cores' no-swizzle layouts, and moving by a voxel moves the start
+// address by 16 bytes: the operand of each of the 27 taps is the same staged tile read from
+// another start address.  In the weight gradient the reduction runs over voxels, so the same
+// layout is the MN-major form of both operands (channels contiguous).  With stride 2 the
+// voxels of a row are stored even ones first, so that a tap's voxels stay consecutive; the
+// input gradient with stride 2 runs as eight kernels' worth of CTAs, one per parity of the
+// input voxel, each with the one to eight taps that reach it.
+// Producer warps gather (8 coalesced loads per 16 staged bytes), convert and store; one warp
+// issues the MMAs; two buffers alternate, handed over by mbarriers.  Every wait on an mbarrier
+// is bounded: past the limit the kernel records an error in `err`, skips the epilogue, and
+// releases its tensor memory.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -35,9 +39,6 @@
 
 namespace pf {
 
-constexpr int kTcRows = 128;   // rows per CTA (MMA M)
-constexpr int kTcKC = 64;      // reduction chunk (4 MMAs of K = 16)
-constexpr int kTcThreads = 128;
 constexpr long long kTcSpin = 1LL << 20;  // try_wait polls before giving up
 
 // ---- descriptors -----------------------------------------------------------------------
@@ -48,10 +49,13 @@ __host__ __device__ constexpr uint64_t umma_smem_desc(uint32_t addr, uint32_t lb
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
 }
-// instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 accumulator, M x N
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
+// (MN-major, no swizzle: the leading offset is between groups of 8 along K, the stride offset
+// between groups of 8 along M or N)
+// instruction descriptor of kind::f16: BF16 A and B, FP32 accumulator, M x N
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N, bool mn_major = false) {
     return (1u << 4)                       // D format F32
            | (1u << 7) | (1u << 10)        // A, B format BF16
+           | (mn_major ? 3u << 15 : 0u)    // A and B MN-major instead of K-major
            | ((uint32_t)(N >> 3) << 17)    // N / 8
            | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
@@ -64,6 +68,8 @@ static bool tc_encodings_match() {
                                                               cute::UMMA::Major::K, cute::UMMA::Major::K>());
     const uint32_t i16 = uint32_t(cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, 128, 16,
                                                               cute::UMMA::Major::K, cute::UMMA::Major::K>());
+    const uint32_t mn = uint32_t(cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, 64, 32,
+                                                             cute::UMMA::Major::MN, cute::UMMA::Major::MN>());
     cute::UMMA::SmemDescriptor d;
     d.desc_ = 0;
     d.start_address_ = (uint16_t)(0x1230 >> 4);
@@ -73,7 +79,7 @@ static bool tc_encodings_match() {
     d.lbo_mode_ = 0;
     d.base_offset_ = 0;
     d.layout_type_ = uint8_t(cute::UMMA::LayoutType::SWIZZLE_NONE);
-    return i64 == umma_idesc_bf16(128, 64) && i16 == umma_idesc_bf16(128, 16) &&
+    return mn == umma_idesc_bf16(64, 32, true) && i64 == umma_idesc_bf16(128, 64) && i16 == umma_idesc_bf16(128, 16) &&
            uint64_t(d) == umma_smem_desc(0x1230, 2048, 128);
 #else
     return true;
@@ -154,170 +160,214 @@ struct ConvTcArgs {
     int X, Y, Z, Xo, Yo, Zo;
 };
 
-// shared memory of one CTA: A0 A1 (rows x chunk) B0 B1 (NP x chunk), 2 mbarriers, TMEM slot
-__device__ __forceinline__ size_t tc_a_bytes() { return (size_t)kTcRows * kTcKC * 2; }
-static size_t tc_smem_bytes(int NP) {
-    return 2 * ((size_t)kTcRows * kTcKC * 2 + (size_t)NP * kTcKC * 2) + 2 * sizeof(uint64_t) + 16;
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Stage 8 consecutive-k values of row `row` of A (rows x 64 chunk) at group g, and the MMA
-// issue/commit of one chunk: shared by the three kernels.
-__device__ __forceinline__ void tc_store_a(uint8_t* sA, int row, int g, uint4 q) {
-    const int slice = g >> 1, half = g & 1;
-    *reinterpret_cast<uint4*>(sA + slice * (kTcRows * 32) + half * (kTcRows * 16) + (row >> 3) * 128 + (row & 7) * 16) = q;
-}
-__device__ __forceinline__ void tc_store_b(uint8_t* sB, int NP, int j, int g, uint4 q) {
-    const int slice = g >> 1, half = g & 1;
-    *reinterpret_cast<uint4*>(sB + slice * (NP * 32) + half * (NP * 16) + (j >> 3) * 128 + (j & 7) * 16) = q;
-}
-__device__ __forceinline__ void tc_issue_chunk(uint32_t tmem, const uint8_t* sA, const uint8_t* sB, int NP,
-                                               uint32_t idesc, long long k0, long long kend, bool first,
-                                               uint64_t* bar) {
-    tc_fence_after();
-    const uint32_t abase = smem_u32(sA), bbase = smem_u32(sB);
+constexpr size_t kTcMaxSmem = 220 * 1024;
+constexpr size_t kTcHalfSmem = 113 * 1024 - 512;  // with the static shared memory, two CTAs per SM
+
+// Tile of one CTA: rows of the product are the voxels q of a TX x 16 x 8 ZH box of the row
+// grid, T = TX ZH accumulators of 128 rows; staged source: LX x LY x LZ voxels from
+// q0 * step + org.
+struct ConvTile {
+    int QX, QY, QZ;            // row grid (largest parity class)
+    int SX, SY, SZ;            // source grid
+    int TX, ZH, ntx, nty, ntz;
+    int LX, LY, LZ, even;      // even: z positions of even offset (0: stored in order)
+    int step, org, ost;        // source step per row voxel, origin; row voxel q is output ost * q + parity
+    int NT, ncols, nsplit;     // columns per CTA, tensor memory columns, column splits
+    int nbuf;                  // staging buffers (1 when one chunk holds all reduction channels)
+};
+
+// shared-memory position of raw z offset r
+__device__ __forceinline__ int tc_zpos(int r, int even) { return even ? (r & 1 ? even + (r >> 1) : r >> 1) : r; }
+
+// 8 values at p, p + stride, ... as BF16 (zeros where !in; the first `cnt` of them): the loads
+// are unconditional (an excluded voxel reads a valid address), so that all are in flight together
+__device__ __forceinline__ uint4 tc_gather8(const float* __restrict__ p, int stride, bool in, int cnt) {
+    float v[8];
+    if (cnt >= 8) {
 #pragma unroll
-    for (int j = 0; j < kTcKC / 16; j++) {
-        if (k0 + j * 16 >= kend) break;
-        const uint64_t da = umma_smem_desc(abase + j * (kTcRows * 32), kTcRows * 16, 128);
-        const uint64_t db = umma_smem_desc(bbase + j * (NP * 32), NP * 16, 128);
-        tc_mma(tmem, da, db, idesc, (!first || j > 0) ? 1u : 0u);
+        for (int j = 0; j < 8; j++) {
+            v[j] = __ldg(p);
+            p += stride;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = j < cnt ? __ldg(p + (long long)j * stride) : 0.f;
     }
-    tc_commit(bar);
+    uint4 q;
+    q.x = in ? pack_bf16(v[0], v[1]) : 0u;
+    q.y = in ? pack_bf16(v[2], v[3]) : 0u;
+    q.z = in ? pack_bf16(v[4], v[5]) : 0u;
+    q.w = in ? pack_bf16(v[6], v[7]) : 0u;
+    return q;
 }
-__device__ __forceinline__ uint32_t tc_setup(uint8_t* smem, int NP, int ncols, uint64_t** bars_out) {
-    const int tid = threadIdx.x, warp = tid >> 5;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * (tc_a_bytes() + (size_t)NP * kTcKC * 2));
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
-    if (warp == 0) {
-        tc_alloc(tslot, (uint32_t)ncols);
+
+constexpr int kTcProd = 256;  // producer threads of the forward / input gradient (8 warps)
+
+constexpr int kTcIssue = 4;    // issuing warps (one thread each; an accumulator has one issuer)
+
+// MODE 0: forward, MODE 1: input gradient.  Warps 0..7 stage and run the epilogue, warps 8..11
+// issue: a single thread needed about 400 cycles per MMA beside the producers, six times what the
+// MMA itself takes.
+template <int MODE>
+__global__ void __launch_bounds__(kTcProd + 32 * kTcIssue, 2) k_conv_tc(ConvTcArgs a, ConvTile t) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t s_full[2], s_empty[2], s_done;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_ntap, s_tw[27], s_ts[27];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NCH = MODE == 0 ? a.Cout : a.Cin, KCH = MODE == 0 ? a.Cin : a.Cout;
+    const int nvox = t.LX * t.LY * t.LZ;
+    const size_t a_bytes = (size_t)nvox * 32, b_bytes = (size_t)27 * 32 * t.NT;
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + t.nbuf * a_bytes;
+    int* s_off = reinterpret_cast<int*>(sB + t.nbuf * b_bytes);
+    const int n = blockIdx.y / t.nsplit, j0 = (int)(blockIdx.y % t.nsplit) * t.NT;
+    const int par = blockIdx.z, px = par & 1, py = (par >> 1) & 1, pz = par >> 2;  // parity class (stride-2 input gradient)
+    const int bz = blockIdx.x % t.ntz, by = (blockIdx.x / t.ntz) % t.nty, bx = blockIdx.x / (t.ntz * t.nty);
+    const int q0x = bx * t.TX, q0y = by * 16, q0z = bz * 8 * t.ZH;
+    const int nchunk = (KCH + 15) / 16, T = t.TX * t.ZH, nis = min(kTcIssue, T);
+    if (warp == 8) {
+        tc_alloc(&s_tmem, (uint32_t)t.ncols);
         tc_relinquish();
     }
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int b = 0; b < 2; b++) {
+            mbar_init(&s_full[b], kTcProd);
+            mbar_init(&s_empty[b], nis);
+        }
+        mbar_init(&s_done, nis);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid == 32) {  // taps: weight index and start offset in the staged tile
+        int k = 0;
+        for (int w = 0; w < 27; w++) {
+            const int tx = w / 9, ty = (w / 3) % 3, tz = w % 3;
+            int dx, dy, dz;
+            if (MODE == 0) {
+                dx = tx, dy = ty, dz = tz;
+            } else if (a.s == 1) {
+                dx = 2 - tx, dy = 2 - ty, dz = 2 - tz;
+            } else {  // input voxel 2q + p takes the taps t with t = p + 1 (mod 2), from q + (p + 1 - t) / 2
+                if (((px + 1 - tx) & 1) || ((py + 1 - ty) & 1) || ((pz + 1 - tz) & 1)) continue;
+                dx = (px + 1 - tx) >> 1, dy = (py + 1 - ty) >> 1, dz = (pz + 1 - tz) >> 1;
+            }
+            s_tw[k] = w;
+            s_ts[k] = (dx * t.LY + dy) * t.LZ + tc_zpos(dz, t.even);
+            k++;
+        }
+        s_ntap = k;
+    }
+    if (tid < kTcProd) {  // source offset of every staged voxel (-1 outside)
+        for (int v = tid; v < nvox; v += kTcProd) {
+            const int row = v / t.LZ, lx = row / t.LY;
+            const int p = v - row * t.LZ, ly = row - lx * t.LY;
+            const int lz = t.even ? (p < t.even ? 2 * p : 2 * (p - t.even) + 1) : p;
+            const int gx = q0x * t.step + t.org + lx, gy = q0y * t.step + t.org + ly, gz = q0z * t.step + t.org + lz;
+            const bool in = gx >= 0 && gy >= 0 && gz >= 0 && gx < t.SX && gy < t.SY && gz < t.SZ;
+            s_off[v] = in ? (gx * t.SY + gy) * t.SZ + gz : -1;
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    *bars_out = bars;
-    return *tslot;
-}
-
-// MODE 0: forward, MODE 1: input gradient
-template <int MODE>
-__global__ void __launch_bounds__(kTcThreads, 1) k_conv_tc(ConvTcArgs a, int NP, int ncols) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    // rows: output voxels (forward) or input voxels (input gradient)
-    const int RX = MODE == 0 ? a.Xo : a.X, RY = MODE == 0 ? a.Yo : a.Y, RZ = MODE == 0 ? a.Zo : a.Z;
-    const long long Vr = (long long)RX * RY * RZ;
-    const int NCH = MODE == 0 ? a.Cout : a.Cin;  // GEMM columns (output channels of the product)
-    const int KCH = MODE == 0 ? a.Cin : a.Cout;  // reduction channels
-    const int K = KCH * 27;
-    const int nchunks = (K + kTcKC - 1) / kTcKC;
-    const int n = blockIdx.y;
-    const size_t a_bytes = tc_a_bytes(), b_bytes = (size_t)NP * kTcKC * 2;
-    auto sA = [&](int buf) { return smem + buf * a_bytes; };
-    auto sB = [&](int buf) { return smem + 2 * a_bytes + buf * b_bytes; };
-    uint64_t* bars;
-    const uint32_t tmem = tc_setup(smem, NP, ncols, &bars);
-
-    const long long r = (long long)blockIdx.x * kTcRows + tid;
-    const bool rv = r < Vr;
-    int rx = 0, ry = 0, rz = 0;
-    if (rv) {
-        rz = (int)(r % RZ);
-        ry = (int)((r / RZ) % RY);
-        rx = (int)(r / ((long long)RZ * RY));
-    }
-    const float* src_n =
-        a.src + (long long)n * KCH * (MODE == 0 ? (long long)a.X * a.Y * a.Z : (long long)a.Xo * a.Yo * a.Zo);
-    const uint32_t idesc = umma_idesc_bf16(kTcRows, NP);
-
-    // operand A[r, k] of this thread's row
-    auto a_val = [&](int k) -> float {
-        if (!rv || k >= K) return 0.f;
-        const int c = k / 27, t = k - c * 27;
-        const int tx = t / 9, ty = (t / 3) % 3, tz = t % 3;
-        if constexpr (MODE == 0) {
-            const int ix = a.s * rx + tx - 1, iy = a.s * ry + ty - 1, iz = a.s * rz + tz - 1;
-            if (ix < 0 || iy < 0 || iz < 0 || ix >= a.X || iy >= a.Y || iz >= a.Z) return 0.f;
-            return __ldg(src_n + (((long long)c * a.X + ix) * a.Y + iy) * a.Z + iz);
-        } else {
-            const int px = rx - tx + 1, py = ry - ty + 1, pz = rz - tz + 1;
-            if (px < 0 || py < 0 || pz < 0 || px % a.s || py % a.s || pz % a.s) return 0.f;
-            const int ox = px / a.s, oy = py / a.s, oz = pz / a.s;
-            if (ox >= a.Xo || oy >= a.Yo || oz >= a.Zo) return 0.f;
-            return __ldg(src_n + (((long long)c * a.Xo + ox) * a.Yo + oy) * a.Zo + oz);
-        }
-    };
-    // operand B[k, j] (j an output channel of the product)
-    auto b_val = [&](int j, int k) -> float {
-        if (j >= NCH || k >= K) return 0.f;
-        if constexpr (MODE == 0) {
-            return __ldg(a.w + (long long)j * K + k);
-        } else {
-            const int co = k / 27, t = k - co * 27;
-            return __ldg(a.w + ((long long)co * a.Cin + j) * 27 + t);
-        }
-    };
-
+    const uint32_t tmem = s_tmem;
+    const int ntap = s_ntap;
     bool ok = true;
-    uint32_t phases = 0u;  // bit b: parity of the next completion of buffer b's barrier
-    for (int c = 0; c < nchunks; c++) {
-        const int buf = c & 1;
-        if (c >= 2) {  // the MMAs of chunk c - 2 read this buffer
-            if (!mbar_wait(&bars[buf], (phases >> buf) & 1u)) ok = false;
-            phases ^= 1u << buf;
+    if (warp < 8) {
+        const long long V = (long long)t.SX * t.SY * t.SZ;
+        const float* src = a.src + (long long)n * KCH * V;
+        for (int c = 0; c < nchunk; c++) {
+            const int b = c & 1;
+            if (c >= 2 && !mbar_wait(&s_empty[b], ((c >> 1) - 1) & 1)) ok = false;
+            uint4* dA = reinterpret_cast<uint4*>(sA + b * a_bytes);
+            for (int h = 0; h < 2; h++) {
+                const int ch0 = c * 16 + h * 8, cnt = KCH - ch0;
+                const float* sc = src + (long long)(cnt > 0 ? ch0 : 0) * V;
+#pragma unroll 2
+                for (int v = tid; v < nvox; v += kTcProd) {
+                    const int off = s_off[v];
+                    dA[h * nvox + v] = tc_gather8(sc + max(off, 0), (int)V, off >= 0, cnt);
+                }
+            }
+            // weights of the chunk, lanes over the taps: (tap, half, column) -> 8 reduction channels
+            uint4* dB = reinterpret_cast<uint4*>(sB + b * b_bytes);
+            if (lane < ntap) {
+                const int wt = s_tw[lane];
+#pragma unroll 2
+                for (int r = warp; r < 2 * t.NT; r += kTcProd / 32) {
+                    const int h = r & 1, j = r >> 1, ch0 = c * 16 + h * 8, cnt = KCH - ch0;
+                    const bool in = j0 + j < NCH;
+                    const int jc = in ? j0 + j : 0, chc = cnt > 0 ? ch0 : 0;
+                    const long long at = MODE == 0 ? (long long)jc * KCH + chc : (long long)chc * a.Cin + jc;
+                    dB[(lane * 2 + h) * t.NT + j] = tc_gather8(a.w + at * 27 + wt, MODE == 0 ? 27 : 27 * a.Cin, in, cnt);
+                }
+            }
+            fence_async_smem();  // the generic-proxy stores become visible to the tensor cores
+            mbar_arrive(&s_full[b]);
         }
-        const int k0 = c * kTcKC;
-#pragma unroll 1
-        for (int g = 0; g < kTcKC / 8; g++) {
-            const int kb = k0 + g * 8;
-            uint4 q;
-            q.x = pack_bf16(a_val(kb + 0), a_val(kb + 1));
-            q.y = pack_bf16(a_val(kb + 2), a_val(kb + 3));
-            q.z = pack_bf16(a_val(kb + 4), a_val(kb + 5));
-            q.w = pack_bf16(a_val(kb + 6), a_val(kb + 7));
-            tc_store_a(sA(buf), tid, g, q);
+    } else if (lane == 0 && warp - 8 < nis) {
+        const uint32_t idesc = umma_idesc_bf16(128, t.NT);
+        // this issuer's accumulators: tiles m0 and m0 + 4
+        const int m0 = warp - 8, m1 = m0 + kTcIssue;
+        auto tile_at = [&](int m) { return (uint64_t)((m / t.ZH) * t.step * t.LY * t.LZ + (m % t.ZH) * 8); };
+        const uint64_t at0 = tile_at(m0), at1 = tile_at(m1) - at0;
+        const uint32_t d0 = tmem + (uint32_t)(m0 * t.NT), d1 = tmem + (uint32_t)(m1 * t.NT);
+        const bool second = m1 < T;
+        for (int c = 0; c < nchunk && ok; c++) {
+            const int b = c & 1;
+            ok = mbar_wait(&s_full[b], (c >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t da0 =
+                umma_smem_desc(smem_u32(sA + b * a_bytes), (uint32_t)nvox * 16, (uint32_t)(t.step * t.LZ * 16)) + at0;
+            uint64_t db = umma_smem_desc(smem_u32(sB + b * b_bytes), (uint32_t)t.NT * 16, 128);
+            uint32_t accum = c ? 1u : 0u;
+#pragma unroll 3
+            for (int k = 0; k < ntap; k++) {
+                const uint64_t da = da0 + (uint64_t)s_ts[k];
+                tc_mma(d0, da, db, idesc, accum);
+                if (second) tc_mma(d1, da + at1, db, idesc, accum);
+                db += (uint64_t)(2 * t.NT);
+                accum = 1u;
+            }
+            tc_commit(&s_empty[b]);
         }
-        for (int idx = tid; idx < NP * (kTcKC / 8); idx += kTcThreads) {
-            const int j = idx / (kTcKC / 8), g = idx % (kTcKC / 8);
-            const int kb = k0 + g * 8;
-            uint4 q;
-            q.x = pack_bf16(b_val(j, kb + 0), b_val(j, kb + 1));
-            q.y = pack_bf16(b_val(j, kb + 2), b_val(j, kb + 3));
-            q.z = pack_bf16(b_val(j, kb + 4), b_val(j, kb + 5));
-            q.w = pack_bf16(b_val(j, kb + 6), b_val(j, kb + 7));
-            tc_store_b(sB(buf), NP, j, g, q);
-        }
-        fence_async_smem();  // the generic-proxy stores become visible to the tensor cores
-        __syncthreads();
-        if (tid == 0) tc_issue_chunk(tmem, sA(buf), sB(buf), NP, idesc, k0, K, c == 0, &bars[buf]);
+        if (ok) tc_commit(&s_done);
     }
-    // the last commit tracks every MMA issued before it
-    const int lb = (nchunks - 1) & 1;
-    if (!mbar_wait(&bars[lb], (phases >> lb) & 1u)) ok = false;
+    __syncwarp();
+    if (!mbar_wait(&s_done, 0)) ok = false;
     tc_fence_after();
     // tcgen05.ld is warp-collective: decide the epilogue for the whole block
     if (__syncthreads_and(ok ? 1 : 0)) {
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < NP; c0 += 16) {
-            float v[16];
-            tc_ld16(trow + (uint32_t)c0, v);
-            if (rv) {
+        if (warp < 8) {
+            const int y = t.ost * (q0y + (warp & 3) * 4 + (lane >> 3)) + py;
+            const int RX = MODE == 0 ? a.Xo : a.X, RY = MODE == 0 ? a.Yo : a.Y, RZ = MODE == 0 ? a.Zo : a.Z;
+            const long long Vr = (long long)RX * RY * RZ;
+            for (int m = warp >> 2; m < T; m += 2) {
+                const int x = t.ost * (q0x + m / t.ZH) + px, z = t.ost * (q0z + (m % t.ZH) * 8 + (lane & 7)) + pz;
+                const bool rv = x < RX && y < RY && z < RZ;
+                float* dst = a.dst + (long long)n * NCH * Vr + ((long long)x * RY + y) * RZ + z;
+                for (int c0 = 0; c0 < t.NT; c0 += 16) {
+                    float v[16];
+                    tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(m * t.NT + c0), v);
+                    if (rv) {
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int ch = c0 + i;
-                    if (ch >= NCH) break;
-                    float* d = a.dst + ((long long)n * NCH + ch) * Vr + r;
-                    if constexpr (MODE == 0) {
-                        float yv = v[i] + __ldg(a.b + ch);
-                        if (a.relu) yv = fmaxf(yv, 0.f);
-                        *d = yv;
-                    } else {
-                        *d = a.accumulate ? *d + v[i] : v[i];
+                        for (int i = 0; i < 16; i++) {
+                            const int ch = j0 + c0 + i;
+                            if (ch >= NCH) break;
+                            float* d = dst + (long long)ch * Vr;
+                            if constexpr (MODE == 0) {
+                                float yv = v[i] + __ldg(a.b + ch);
+                                if (a.relu) yv = fmaxf(yv, 0.f);
+                                *d = yv;
+                            } else {
+                                *d = a.accumulate ? *d + v[i] : v[i];
+                            }
+                        }
                     }
                 }
             }
@@ -327,99 +377,179 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv_tc(ConvTcArgs a, int NP,
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, (uint32_t)ncols);
+    if (warp == 8) tc_dealloc(tmem, (uint32_t)t.ncols);
 }
 
-// Weight gradient: the voxels are split into ranges of kTcWSplit; CTA (row tile, range)
-// writes its partial D to part[range][co][m] and k_conv_tc_wsum adds the ranges in order.
-constexpr int kTcWSplit = 4096;
+// Weight gradient.  The output voxels are cut into tiles of TX x 16 x 8, the tiles into `nsplit`
+// ranges; CTA (range, tap group, input-channel tile, column split) accumulates its taps'
+// 64 x NT products (row: input channel, after them one row of ones that gives the bias
+// gradient; column: output channel) over its range in tensor memory and writes them to
+// part[range][co][ci * 27 + t]; k_conv_tc_wsum adds the ranges in order.
+constexpr int kTcWSplit = 4096;  // voxels per range (sets the workspace)
+constexpr int kTcWProd = 512;
 
-__global__ void __launch_bounds__(kTcThreads, 1) k_conv_tc_wgrad(ConvTcArgs a, int NP, int ncols, int Mtot,
-                                                                 float* __restrict__ part) {
+struct ConvWTile {
+    int TX, ntx, nty, ntz;
+    int LX, LY, LZ, even;
+    int np;                // planes of 8 input channels per CTA (the plane of ones follows)
+    int nci;               // input-channel tiles
+    int NT, nco, TG, ntg;  // columns per CTA and splits, taps per CTA and groups
+    int ncols, nsplit;
+};
+
+constexpr int kTcWTaps = 7;  // taps of one issuing thread: ceil(27 / 4)
+
+__global__ void __launch_bounds__(kTcWProd + 32 * kTcIssue, 1) k_conv_tc_wgrad(ConvTcArgs a, ConvWTile t, float* __restrict__ part) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const long long Vo = (long long)a.Xo * a.Yo * a.Zo, Vi = (long long)a.X * a.Y * a.Z;
-    const long long Ktot = (long long)a.N * Vo;
-    const long long kbeg = (long long)blockIdx.y * kTcWSplit;
-    const long long kend = kbeg + kTcWSplit < Ktot ? kbeg + kTcWSplit : Ktot;
-    const int nchunks = (int)((kend - kbeg + kTcKC - 1) / kTcKC);
-    const size_t a_bytes = tc_a_bytes(), b_bytes = (size_t)NP * kTcKC * 2;
-    auto sA = [&](int buf) { return smem + buf * a_bytes; };
-    auto sB = [&](int buf) { return smem + 2 * a_bytes + buf * b_bytes; };
-    uint64_t* bars;
-    const uint32_t tmem = tc_setup(smem, NP, ncols, &bars);
-    // this thread's row: (ci, tap), the bias row, or padding
-    const int m = blockIdx.x * kTcRows + tid;
-    const int M = 27 * a.Cin;
-    const bool is_w = m < M, is_b = m == M;
-    const int ci = is_w ? m / 27 : 0, t = is_w ? m % 27 : 0;
-    const int tx = t / 9, ty = (t / 3) % 3, tz = t % 3;
-    const uint32_t idesc = umma_idesc_bf16(kTcRows, NP);
-
-    auto a_val = [&](long long k) -> float {
-        if (k >= kend || !(is_w || is_b)) return 0.f;
-        if (is_b) return 1.f;
-        const int n = (int)(k / Vo);
-        const long long o = k - (long long)n * Vo;
-        const int oz = (int)(o % a.Zo), oy = (int)((o / a.Zo) % a.Yo), ox = (int)(o / ((long long)a.Zo * a.Yo));
-        const int ix = a.s * ox + tx - 1, iy = a.s * oy + ty - 1, iz = a.s * oz + tz - 1;
-        if (ix < 0 || iy < 0 || iz < 0 || ix >= a.X || iy >= a.Y || iz >= a.Z) return 0.f;
-        return __ldg(a.src + ((long long)n * a.Cin + ci) * Vi + ((long long)ix * a.Y + iy) * a.Z + iz);
-    };
-    auto b_val = [&](int co, long long k) -> float {
-        if (co >= a.Cout || k >= kend) return 0.f;
-        const int n = (int)(k / Vo);
-        const long long o = k - (long long)n * Vo;
-        return __ldg(a.w + ((long long)n * a.Cout + co) * Vo + o);  // dy
-    };
-
-    bool ok = true;
-    uint32_t phases = 0u;
-    for (int c = 0; c < nchunks; c++) {
-        const int buf = c & 1;
-        if (c >= 2) {
-            if (!mbar_wait(&bars[buf], (phases >> buf) & 1u)) ok = false;
-            phases ^= 1u << buf;
-        }
-        const long long k0 = kbeg + (long long)c * kTcKC;
-#pragma unroll 1
-        for (int g = 0; g < kTcKC / 8; g++) {
-            const long long kb = k0 + g * 8;
-            uint4 q;
-            q.x = pack_bf16(a_val(kb + 0), a_val(kb + 1));
-            q.y = pack_bf16(a_val(kb + 2), a_val(kb + 3));
-            q.z = pack_bf16(a_val(kb + 4), a_val(kb + 5));
-            q.w = pack_bf16(a_val(kb + 6), a_val(kb + 7));
-            tc_store_a(sA(buf), tid, g, q);
-        }
-        for (int idx = tid; idx < NP * (kTcKC / 8); idx += kTcThreads) {
-            const int j = idx / (kTcKC / 8), g = idx % (kTcKC / 8);
-            const long long kb = k0 + g * 8;
-            uint4 q;
-            q.x = pack_bf16(b_val(j, kb + 0), b_val(j, kb + 1));
-            q.y = pack_bf16(b_val(j, kb + 2), b_val(j, kb + 3));
-            q.z = pack_bf16(b_val(j, kb + 4), b_val(j, kb + 5));
-            q.w = pack_bf16(b_val(j, kb + 6), b_val(j, kb + 7));
-            tc_store_b(sB(buf), NP, j, g, q);
-        }
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) tc_issue_chunk(tmem, sA(buf), sB(buf), NP, idesc, k0, kend, c == 0, &bars[buf]);
+    __shared__ uint64_t s_full[2], s_empty[2], s_done;
+    __shared__ uint32_t s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nrow = t.LX * t.LY, nvox = nrow * t.LZ, np1 = t.np + 1, RP = np1 * t.LZ;  // row pitch, 16-byte units
+    const int nvd = t.TX * 128;
+    const size_t a_bytes = (size_t)nrow * RP * 16, b_bytes = (size_t)(t.NT / 8) * nvd * 16;
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + 2 * a_bytes;
+    int2* s_tab = reinterpret_cast<int2*>(sB + 2 * b_bytes);  // two tables of nvox
+    const int range = blockIdx.x, tg = blockIdx.y % t.ntg, cot = blockIdx.y / t.ntg;
+    const int co0 = cot * t.NT, ci0 = blockIdx.z * t.np * 8;
+    const int tap0 = tg * t.TG, ntap = min(t.TG, 27 - tap0);
+    const long long ntile = (long long)a.N * t.ntx * t.nty * t.ntz;
+    const long long tb = ntile * range / t.nsplit, te = ntile * (range + 1) / t.nsplit;
+    if (warp == 16) {
+        tc_alloc(&s_tmem, (uint32_t)t.ncols);
+        tc_relinquish();
     }
-    const int lb = (nchunks - 1) & 1;
-    if (!mbar_wait(&bars[lb], (phases >> lb) & 1u)) ok = false;
+    if (tid == 0) {
+        for (int b = 0; b < 2; b++) {
+            mbar_init(&s_full[b], kTcWProd);
+            mbar_init(&s_empty[b], kTcIssue);
+        }
+        mbar_init(&s_done, kTcIssue);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid < kTcWProd) {  // the planes of ones stay as they are
+        const uint4 one = {0x3f80u, 0u, 0u, 0u};
+        for (int v = tid; v < 2 * nvox; v += kTcWProd) {
+            const int b = v >= nvox, q = v - b * nvox, row = q / t.LZ;
+            *reinterpret_cast<uint4*>(sA + b * a_bytes + ((size_t)row * RP + t.np * t.LZ + q - row * t.LZ) * 16) = one;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
     tc_fence_after();
-    if (__syncthreads_and(ok ? 1 : 0)) {
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < NP; c0 += 16) {
-            float v[16];
-            tc_ld16(trow + (uint32_t)c0, v);
-            if (m < Mtot) {
+    const uint32_t tmem = s_tmem;
+    bool ok = true;
+    if (warp < 16) {
+        const long long Vi = (long long)a.X * a.Y * a.Z, Vo = (long long)a.Xo * a.Yo * a.Zo;
+        int c = 0;
+        for (long long tl = tb; tl < te; tl++, c++) {
+            const int b = c & 1;
+            int r = (int)(tl % (t.ntx * t.nty * t.ntz));
+            const int n = (int)(tl / (t.ntx * t.nty * t.ntz));
+            const int oz0 = (r % t.ntz) * 8, oy0 = (r / t.ntz) % t.nty * 16, ox0 = r / (t.ntz * t.nty) * t.TX;
+            int2* tab = s_tab + b * nvox;
+            for (int v = tid; v < nvox; v += kTcWProd) {
+                const int row = v / t.LZ, lx = row / t.LY;
+                const int p = v - row * t.LZ, ly = row - lx * t.LY;
+                const int lz = t.even ? (p < t.even ? 2 * p : 2 * (p - t.even) + 1) : p;
+                const int gx = ox0 * a.s - 1 + lx, gy = oy0 * a.s - 1 + ly, gz = oz0 * a.s - 1 + lz;
+                const bool in = gx >= 0 && gy >= 0 && gz >= 0 && gx < a.X && gy < a.Y && gz < a.Z;
+                tab[v] = make_int2(in ? (gx * a.Y + gy) * a.Z + gz : -1, row * RP + p);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kTcWProd) : "memory");  // the table, among the producers
+            if (c >= 2 && !mbar_wait(&s_empty[b], ((c >> 1) - 1) & 1)) ok = false;
+            uint8_t* dA = sA + b * a_bytes;
+            const float* x = a.src + (long long)n * a.Cin * Vi;
+            int h = 0, v = tid;
+            while (v >= nvox) v -= nvox, h++;
+#pragma unroll 2
+            for (int it = tid; it < t.np * nvox; it += kTcWProd) {
+                const int2 e = tab[v];
+                const int ch0 = ci0 + h * 8, cnt = a.Cin - ch0;
+                *reinterpret_cast<uint4*>(dA + ((size_t)e.y + h * t.LZ) * 16) =
+                    tc_gather8(x + (long long)(cnt > 0 ? ch0 : 0) * Vi + max(e.x, 0), (int)Vi, e.x >= 0, cnt);
+                v += kTcWProd;
+                while (v >= nvox) v -= nvox, h++;
+            }
+            uint8_t* dB = sB + b * b_bytes;
+            const float* dy = a.w + (long long)n * a.Cout * Vo;
+            for (int it = tid; it < (t.NT / 8) * nvd; it += kTcWProd) {
+                const int g = it / nvd, q = it - g * nvd;
+                const int ox = ox0 + (q >> 7), oy = oy0 + ((q >> 3) & 15), oz = oz0 + (q & 7);
+                const bool in = ox < a.Xo && oy < a.Yo && oz < a.Zo;
+                const int ch0 = co0 + g * 8, cnt = a.Cout - ch0;
+                *reinterpret_cast<uint4*>(dB + (size_t)it * 16) = tc_gather8(
+                    dy + (long long)(cnt > 0 ? ch0 : 0) * Vo + (in ? (ox * a.Yo + oy) * a.Zo + oz : 0), (int)Vo, in, cnt);
+            }
+            fence_async_smem();
+            mbar_arrive(&s_full[b]);
+        }
+    } else if (lane == 0) {
+        const uint32_t idesc = umma_idesc_bf16(64, t.NT, true);
+        // this issuer's taps: every fourth; their start offsets and accumulators
+        const int is = warp - kTcWProd / 32;
+        uint32_t off[kTcWTaps];
+        int nk = 0;
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int co = c0 + i;
-                    if (co >= a.Cout) break;
-                    part[((long long)blockIdx.y * a.Cout + co) * Mtot + m] = v[i];
+        for (int i = 0; i < kTcWTaps; i++) {
+            const int k = is + i * kTcIssue, w = tap0 + k, tx = w / 9, ty = (w / 3) % 3, tz = w % 3;
+            off[i] = (uint32_t)((tx * t.LY + ty) * RP + tc_zpos(tz, t.even));
+            if (k < ntap) nk++;
+        }
+        const uint32_t d0 = tmem + (uint32_t)(is * t.NT), dstep = (uint32_t)(kTcIssue * t.NT);
+        int c = 0;
+        for (long long tl = tb; tl < te && ok; tl++, c++) {
+            const int b = c & 1;
+            ok = mbar_wait(&s_full[b], (c >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t da0 = umma_smem_desc(smem_u32(sA + b * a_bytes), (uint32_t)(a.s * RP * 16), (uint32_t)(t.LZ * 16));
+            uint64_t db = umma_smem_desc(smem_u32(sB + b * b_bytes), 128, (uint32_t)(nvd * 16));
+            uint32_t accum = c ? 1u : 0u;
+            for (int x = 0; x < t.TX; x++) {
+                uint64_t da = da0 + (uint64_t)(x * a.s * t.LY * RP);
+                for (int y = 0; y < 16; y += 2) {  // 16 voxels: two rows of 8
+                    uint32_t d = d0;
+#pragma unroll
+                    for (int i = 0; i < kTcWTaps; i++) {
+                        if (i < nk) tc_mma(d, da + off[i], db, idesc, accum);
+                        d += dstep;
+                    }
+                    da += (uint64_t)(2 * a.s * RP);
+                    db += 16;
+                    accum = 1u;
+                }
+            }
+            tc_commit(&s_empty[b]);
+        }
+        if (ok) tc_commit(&s_done);
+    }
+    __syncwarp();
+    if (te > tb && !mbar_wait(&s_done, 0)) ok = false;
+    tc_fence_after();
+    const int Mtot = 27 * a.Cin + 1;
+    if (__syncthreads_and(ok ? 1 : 0)) {
+        // 64-row accumulators: rows 16 q .. 16 q + 15 lie in lanes 32 q .. 32 q + 15
+        if (warp < 16) {
+            const int q = warp & 3, row = q * 16 + lane, ci = ci0 + row;
+            for (int k = warp >> 2; k < ntap; k += 4) {
+                const int tap = tap0 + k;
+                for (int c0 = 0; c0 < t.NT; c0 += 16) {
+                    float v[16];
+                    tc_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(k * t.NT + c0), v);
+                    int m = -1;
+                    if (lane < 16) {
+                        if (row < t.np * 8 && ci < a.Cin) m = ci * 27 + tap;
+                        if (row == t.np * 8 && tap == 13 && blockIdx.z == 0) m = Mtot - 1;
+                    }
+                    if (m >= 0) {
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            const int co = co0 + c0 + i;
+                            if (co >= a.Cout) break;
+                            part[((long long)range * a.Cout + co) * Mtot + m] = te > tb ? v[i] : 0.f;
+                        }
+                    }
                 }
             }
         }
@@ -428,17 +558,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv_tc_wgrad(ConvTcArgs a, i
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, (uint32_t)ncols);
+    if (warp == 16) tc_dealloc(tmem, (uint32_t)t.ncols);
 }
 
-// dw[co, ci, t] = sum over ranges of part[range][co][ci*27 + t]; db[co] from the ones row
-__global__ void k_conv_tc_wsum(const float* __restrict__ part, int nsplit, int Cout, int Mtot, float* __restrict__ dw,
-                               float* __restrict__ db) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)Cout * Mtot) return;
-    const int co = (int)(i / Mtot), m = (int)(i - (long long)co * Mtot);
+// dw[co, ci, t] = sum over ranges of part[range][co][ci*27 + t]; db[co] from the ones row.
+// Warp g of a block adds every eighth range for 32 outputs, then the eight sums in order (one
+// thread per output over all ranges waited on 16 rounds of loads: 35 us for 128 ranges).
+__global__ void __launch_bounds__(256) k_conv_tc_wsum(const float* __restrict__ part, int nsplit, int Cout, int Mtot,
+                                                      float* __restrict__ dw, float* __restrict__ db) {
+    __shared__ float s_p[8][32];
+    const int g = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const long long tot = (long long)Cout * Mtot, i = (long long)blockIdx.x * 32 + l;
     float s = 0.f;
-    for (int r = 0; r < nsplit; r++) s += part[((long long)r * Cout + co) * Mtot + m];
+    if (i < tot) {
+#pragma unroll 8
+        for (int r = g; r < nsplit; r += 8) s += part[r * tot + i];
+    }
+    s_p[g][l] = s;
+    __syncthreads();
+    if (g != 0 || i >= tot) return;
+#pragma unroll
+    for (int q = 1; q < 8; q++) s += s_p[q][l];
+    const int co = (int)(i / Mtot), m = (int)(i - (long long)co * Mtot);
     if (m < Mtot - 1)
         dw[(long long)co * (Mtot - 1) + m] = s;
     else if (db)
@@ -451,25 +592,72 @@ static int tc_ncols(int NP) {
     return c;
 }
 
-static int tc_check(int NP) {
-    if (NP > 256) return fail(PF_UNSUPPORTED, "tensor-core conv: at most 256 output channels");
+static int tc_check() {
     static const bool enc_ok = tc_encodings_match();
     if (!enc_ok) return fail(PF_UNSUPPORTED, "tensor-core conv: descriptor encoding check failed");
     return PF_OK;
+}
+
+// staged extent along an axis for n row voxels
+static int tc_extent(int mode, int s, int n) { return mode == 0 ? s * (n - 1) + 3 : s == 1 ? n + 2 : n + 1; }
+
+static size_t tc_conv_smem(const ConvTile& t) {
+    const size_t nvox = (size_t)t.LX * t.LY * t.LZ;
+    return t.nbuf * (nvox * 32 + (size_t)27 * 32 * t.NT) + nvox * sizeof(int);
 }
 
 template <int MODE>
 static int launch_conv_tc(const ConvTcArgs& a, cudaStream_t st) {
     const int NCH = MODE == 0 ? a.Cout : a.Cin;
     const int NP = (NCH + 15) / 16 * 16;
-    int s = tc_check(NP);
+    if (NP > 256) return fail(PF_UNSUPPORTED, "tensor-core conv: at most 256 output channels");
+    int s = tc_check();
     if (s) return s;
-    const long long Vr = MODE == 0 ? (long long)a.Xo * a.Yo * a.Zo : (long long)a.X * a.Y * a.Z;
-    const size_t smem = tc_smem_bytes(NP);
-    PF_CUDA(cudaFuncSetAttribute(k_conv_tc<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)((Vr + kTcRows - 1) / kTcRows), (unsigned)a.N);
+    ConvTile t;
+    const bool half = MODE == 1 && a.s == 2;  // one CTA class per parity of the input voxel
+    t.QX = MODE == 0 ? a.Xo : half ? (a.X + 1) / 2 : a.X;
+    t.QY = MODE == 0 ? a.Yo : half ? (a.Y + 1) / 2 : a.Y;
+    t.QZ = MODE == 0 ? a.Zo : half ? (a.Z + 1) / 2 : a.Z;
+    t.SX = MODE == 0 ? a.X : a.Xo;
+    t.SY = MODE == 0 ? a.Y : a.Yo;
+    t.SZ = MODE == 0 ? a.Z : a.Zo;
+    t.step = MODE == 0 ? a.s : 1;
+    t.org = half ? 0 : -1;
+    t.ost = half ? 2 : 1;
+    // columns: equal splits of at most 64, so that the weights of a chunk fit beside the voxels
+    t.nsplit = (NP + 63) / 64;
+    t.NT = (NP / 16 + t.nsplit - 1) / t.nsplit * 16;
+    t.nbuf = (MODE == 0 ? a.Cin : a.Cout) > 16 ? 2 : 1;
+    // tile: the largest of up to 8 accumulators that leaves two CTAs per SM (tensor memory,
+    // shared memory) and at least two CTAs for every SM; else the smallest
+    long long best = -1;
+    ConvTile pick = t;
+    for (int TX = 1; TX <= 4; TX *= 2)
+        for (int ZH = 1; ZH <= 2; ZH++) {
+            ConvTile c = t;
+            c.TX = TX;
+            c.ZH = ZH;
+            c.LX = tc_extent(MODE, a.s, TX);
+            c.LY = tc_extent(MODE, a.s, 16);
+            c.LZ = tc_extent(MODE, a.s, 8 * ZH);
+            c.even = t.step == 2 ? (c.LZ + 1) / 2 : 0;
+            c.ntx = (t.QX + TX - 1) / TX;
+            c.nty = (t.QY + 15) / 16;
+            c.ntz = (t.QZ + 8 * ZH - 1) / (8 * ZH);
+            const long long ctas = (long long)c.ntx * c.nty * c.ntz * a.N * t.nsplit * (half ? 8 : 1);
+            const bool two = TX * ZH * t.NT <= 256 && tc_conv_smem(c) <= kTcHalfSmem;
+            const bool fits = TX * ZH * t.NT <= 512 && tc_conv_smem(c) <= kTcMaxSmem;
+            const long long score = !fits ? -2 : ctas >= 2 * kNumSM ? (two ? 100 : 0) + TX * ZH * 4 + ZH : 0;
+            if (score > best) best = score, pick = c;
+        }
+    if (best < 0) return fail(PF_UNSUPPORTED, "tensor-core conv: no tile fits");
+    t = pick;
+    t.ncols = tc_ncols(t.TX * t.ZH * t.NT);
+    const size_t smem = tc_conv_smem(t);
+    PF_CUDA(cudaFuncSetAttribute(k_conv_tc<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcMaxSmem));
+    dim3 grid((unsigned)(t.ntx * t.nty * t.ntz), (unsigned)(a.N * t.nsplit), half ? 8u : 1u);
     pf::count_launch();
-    k_conv_tc<MODE><<<grid, kTcThreads, smem, st>>>(a, NP, tc_ncols(NP));
+    k_conv_tc<MODE><<<grid, kTcProd + 32 * kTcIssue, smem, st>>>(a, t);
     PF_LAUNCH_CHECK("tensor-core conv launch");
     return PF_OK;
 }
@@ -514,21 +702,52 @@ extern "C" int pf_cnn_conv3d_bwd_weight_tc(const float* x, const float* dy, int 
         (stride != 1 && stride != 2))
         return fail(PF_BAD_ARG, "pf_cnn_conv3d_bwd_weight_tc: bad argument");
     const int NP = (Cout + 15) / 16 * 16;
-    int s = tc_check(NP);
+    if (NP > 256) return fail(PF_UNSUPPORTED, "tensor-core conv: at most 256 output channels");
+    int s = tc_check();
     if (s) return s;
     ConvTcArgs a = {x, dy, nullptr, dw, err, N, Cin, Cout, stride, 0, 0, X, Y, Z,
                     out_ext(X, stride), out_ext(Y, stride), out_ext(Z, stride)};
     const long long Ktot = (long long)N * a.Xo * a.Yo * a.Zo;
     const int nsplit = (int)((Ktot + kTcWSplit - 1) / kTcWSplit);
     const int Mtot = 27 * Cin + 1;
-    const size_t smem = tc_smem_bytes(NP);
+    // input-channel tiles of at most 56 (7 planes and the ones: 64 rows), the largest with which
+    // two buffers of a tile of two or one x planes fit
+    ConvWTile t;
+    t.nco = (NP + 63) / 64;
+    t.NT = (NP / 16 + t.nco - 1) / t.nco * 16;
+    t.TG = 512 / t.NT < 27 ? 512 / t.NT : 27;
+    t.ntg = (27 + t.TG - 1) / t.TG;
+    t.ncols = tc_ncols((t.TG < 27 ? t.TG : 27) * t.NT);
+    t.nsplit = nsplit;
+    t.LY = stride * 15 + 3;
+    t.LZ = stride * 7 + 3;
+    t.even = stride == 2 ? 9 : 0;
+    const int planes = (Cin + 7) / 8;
+    size_t smem = 0;
+    bool found = false;
+    for (int parts = 1; parts <= planes && !found; parts++) {
+        t.np = (planes + parts - 1) / parts;
+        if (t.np > 7) continue;
+        for (int TX = 2; TX >= 1 && !found; TX--) {
+            t.TX = TX;
+            t.LX = stride * (TX - 1) + 3;
+            const size_t vox = (size_t)t.LX * t.LY * t.LZ;
+            smem = 2 * (vox * (t.np + 1) * 16 + (size_t)(t.NT / 8) * TX * 128 * 16 + vox * sizeof(int2));
+            found = smem <= kTcMaxSmem;
+        }
+    }
+    if (!found) return fail(PF_UNSUPPORTED, "tensor-core conv: no tile fits");
+    t.nci = (planes + t.np - 1) / t.np;
+    t.ntx = (a.Xo + t.TX - 1) / t.TX;
+    t.nty = (a.Yo + 15) / 16;
+    t.ntz = (a.Zo + 7) / 8;
     cudaStream_t st = as_stream(stream);
-    PF_CUDA(cudaFuncSetAttribute(k_conv_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PF_CUDA(cudaFuncSetAttribute(k_conv_tc_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcMaxSmem));
     pf::count_launch(2);
-    k_conv_tc_wgrad<<<dim3((unsigned)((Mtot + kTcRows - 1) / kTcRows), (unsigned)nsplit), kTcThreads, smem, st>>>(
-        a, NP, tc_ncols(NP), Mtot, work);
+    k_conv_tc_wgrad<<<dim3((unsigned)nsplit, (unsigned)(t.ntg * t.nco), (unsigned)t.nci), kTcWProd + 32 * kTcIssue, smem, st>>>(a, t,
+                                                                                                                   work);
     const long long nt = (long long)Cout * Mtot;
-    k_conv_tc_wsum<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(work, nsplit, Cout, Mtot, dw, db);
+    k_conv_tc_wsum<<<(unsigned)((nt + 31) / 32), 256, 0, st>>>(work, nsplit, Cout, Mtot, dw, db);
     PF_LAUNCH_CHECK("tensor-core conv weight gradient launch");
     return PF_OK;
 }

@@ -114,3 +114,36 @@ def test_oc_sequences(lib, n, kind):
         assert np.abs(got - ref).max() < 2e-8
     late, _ = _oc(lib, x, df, dg, vf, move, wait=False)
     assert np.array_equal(late, got)
+
+
+@pytest.mark.parametrize("shape,co,stride", [
+    ((1, 1, 1, 1, 1), 1, 1), ((1, 17, 2, 16, 8), 17, 1), ((2, 57, 5, 17, 9), 65, 1), ((1, 64, 3, 33, 17), 48, 2),
+    ((2, 16, 16, 32, 32), 16, 1), ((8, 8, 32, 16, 16), 16, 1), ((1, 130, 4, 5, 20), 130, 1), ((1, 33, 1, 2, 3), 20, 2),
+    ((3, 16, 18, 20, 34), 32, 2)])
+def test_conv_tiles(lib, shape, co, stride):
+    # tile edges along each axis, channel chunks of 16 with a remainder, column splits, several
+    # input-channel tiles; operands representable in BF16, so only the FP32 accumulation differs
+    # from float64 (sums of up to 27 * 130 products or 12,000 voxels: 1e-5 of the largest entry)
+    N_, ci, X, Y, Z = shape
+    g = torch.Generator(device="cuda").manual_seed(7)
+    def bf(*s):
+        return torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16).to(torch.float32)
+    x, w, b = bf(*shape), bf(co, ci, 3, 3, 3), torch.randn(co, generator=g, device="cuda")
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    ref = torch.nn.functional.conv3d(xd, wd, b.double(), stride=stride, padding=1)
+    dy = bf(*ref.shape)
+    gx, gw = torch.autograd.grad(ref, (xd, wd), dy.double())
+    L = lib.load()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    y, dx = torch.full_like(dy, np.nan), torch.full_like(x, np.nan)
+    dw, db = torch.full_like(w, np.nan), torch.full_like(b, np.nan)
+    nw = int(L.pf_cnn_conv3d_bwd_weight_tc_workspace(N_, ci, X, Y, Z, co, stride))
+    work = torch.full((nw,), np.nan, dtype=torch.float32, device="cuda")
+    P = lib.ptr
+    lib.check(L.pf_cnn_conv3d_fwd_tc(P(x), N_, ci, X, Y, Z, P(w), P(b), co, stride, 0, P(y), P(err), lib.stream()))
+    lib.check(L.pf_cnn_conv3d_bwd_data_tc(P(dy), N_, ci, X, Y, Z, P(w), co, stride, 0, P(dx), P(err), lib.stream()))
+    lib.check(L.pf_cnn_conv3d_bwd_weight_tc(P(x), P(dy), N_, ci, X, Y, Z, co, stride, P(dw), P(db), P(work), P(err),
+                                            lib.stream()))
+    assert int(err.item()) == 0
+    for got, want in ((y, ref), (dx, gx), (dw, gw), (db, dy.double().sum(dim=(0, 2, 3, 4)))):
+        assert rel(N(got), N(want)) < 1e-5
