@@ -147,3 +147,49 @@ def test_conv_tiles(lib, shape, co, stride):
     assert int(err.item()) == 0
     for got, want in ((y, ref), (dx, gx), (dw, gw), (db, dy.double().sum(dim=(0, 2, 3, 4)))):
         assert rel(N(got), N(want)) < 1e-5
+
+
+@pytest.mark.parametrize("nel", [(1, 1), (3, 2), (2, 9), (60, 20), (20, 60), (33, 45), (45, 45), (120, 40), (300, 5), (46, 46),
+                                 (1, 1, 1), (20, 1, 1), (2, 9, 2), (3, 3, 30), (4, 3, 3), (6, 5, 5)])
+def test_direct_band(lib, nel):
+    # banded and dense route, either axis the longest, windows and halves of every small size.
+    # Cholesky's backward error is a small multiple of (band width) * eps of |K| |x|: 1e-13
+    from conftest import unit_K0
+    dim = len(nel)
+    K0 = unit_K0(dim)
+    rng = np.random.default_rng(sum(nel))
+    ndof = O.n_nodes(nel) * dim
+    E = rng.uniform(0.05, 1.0, O.n_elem(nel))
+    # the nodes of the x = 0 face, and a few single DOFs
+    nx = nel[0] + 1
+    node = np.arange(O.n_nodes(nel))
+    ix = (node // (nel[2] + 1 if dim == 3 else 1)) % nx
+    cons = np.unique(np.concatenate([(node[ix == 0][:, None] * dim + np.arange(dim)).reshape(-1),
+                                     rng.integers(0, ndof, 3)]))
+    b = rng.standard_normal(ndof)
+    free = np.setdiff1d(np.arange(ndof), cons).astype(np.int32)
+    d2f = np.full(ndof, -1, dtype=np.int32)
+    d2f[free] = np.arange(len(free), dtype=np.int32)
+    L = lib.load()
+    grid, op, d = lib.make_grid(nel), ctypes.c_void_p(), ctypes.c_void_p()
+    K0c = np.ascontiguousarray(K0)
+    lib.check(L.pf_op_create(ctypes.byref(grid), K0c.ctypes.data, ctypes.byref(op)))
+    lib.check(L.pf_direct_create(op, ctypes.byref(d)))
+    Et, ft, dt, bt = T(E), T(free, torch.int32), T(d2f, torch.int32), T(b)
+    x = torch.full_like(bt, np.nan)
+    for _ in range(2):
+        lib.check(L.pf_direct_solve_f64(d, lib.ptr(Et), lib.ptr(ft), lib.ptr(dt), len(free), lib.ptr(bt), lib.ptr(x),
+                                        lib.stream()))
+    xs = N(x)
+    assert np.array_equal(xs[cons], b[cons])
+    u = xs.copy()
+    u[cons] = 0.0
+    r = (O.matvec(nel, K0, E, u) - b)[free]
+    norm = 2 ** dim * np.abs(K0).sum(axis=1).max()
+    assert np.linalg.norm(r) < 1e-13 * (norm * np.linalg.norm(u) + np.linalg.norm(b))
+    # a stiffness that is not positive definite is reported
+    Et[: len(E) // 2 + 1] = -1.0
+    assert L.pf_direct_solve_f64(d, lib.ptr(Et), lib.ptr(ft), lib.ptr(dt), len(free), lib.ptr(bt), lib.ptr(x),
+                                 lib.stream()) == lib.PF_FACTOR_FAILED
+    L.pf_direct_destroy(d)
+    L.pf_op_destroy(op)
