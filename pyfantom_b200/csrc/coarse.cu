@@ -17,16 +17,16 @@
 // and no coefficient traffic, where the assembled stencil streams 126 coefficients per
 // coarse node.
 //
-// Coarse elements with a constrained fine node ("dirty": their Z-masked children) keep an
-// explicit Walsh-basis matrix: every coefficient pair (I, J) of the dirty part of A^ (the
-// masked children of all dirty elements containing I and J) is assigned to the first dirty
-// element (in element order) that contains both I and J, so the dirty matrices sum to
-// exactly that part.  A dirty element is marked by Ehat_0 = -(index + 1) (Ehat_0 = sum E > 0
-// otherwise), confirmed against the dirty list.  The identity rows Phat^T (I - Z) Phat are
-// applied per coarse node in the physical basis (27 neighbours per component) by the owner
-// of the node: inside a Walsh-basis matrix their O(1) entries would be mixed with the
-// O(E_min) stiffness of void children, which FP32 cannot resolve (SIMP densities reach
-// 1e-9 of the solid at a clamped face).
+// Coarse elements with a constrained fine node ("dirty") have Z-masked children, and the
+// identity rows Phat^T (I - Z) Phat reach the same elements' corners: the rows of these corner
+// nodes are taken from the assembled level-1 stencil (which the setup forms for the deeper
+// levels) into a compact table.  The march skips them, so what it computes for dirty elements
+// (from their unmasked children) is never used, and the warps of all blocks share them out:
+// a clamped face puts thousands of them into a few tile columns.  (Explicit 24 x 24 matrices
+// inside the march held those columns' blocks back: 53.9 us per FP32 level-1 product of
+// 256x128x128 with a clamped face, 30.0 us without one.)  The stiffness rows stay in the
+// physical basis, where FP32 resolves the O(E_min) stiffness of void children beside the O(1)
+// identity rows to the same relative error as the stencil; in the Walsh basis they would mix.
 //
 // The matvec is an x-march like the fine one (csrc/elemop.cu): warps cover element rows in
 // y, lanes element columns in z, the element's Walsh transform is formed from the two
@@ -149,14 +149,14 @@ int coarse_factorise(const Op* op, double* coef /* [150] */) {
 }
 
 // ---------------------------------------------------------------------------------------
-// setup: dirty-element list, Ehat, dirty Walsh matrices
+// setup: Ehat, rows of the nodes next to constraints
 // ---------------------------------------------------------------------------------------
 constexpr int kScanThreads = 1024;  // flags per block of the compaction
 
 // Stream compaction of a flag array in index order, in two passes: block b counts the
 // flags of items [1024 b, 1024 (b + 1)); then every block adds the counts of the blocks
-// before it and places its items with a ballot scan.  map[i] = rank of item i among the
-// flagged items (or -1), list[rank] = i (rank < cap), *count = number of flagged items.
+// before it and places its items with a ballot scan.  list[rank] = i (rank < cap; list may be
+// NULL), *count = number of flagged items.
 __global__ void __launch_bounds__(kScanThreads) k_flag_count(long long n, const uint8_t* __restrict__ flag,
                                                              int* __restrict__ bcount) {
     const long long i = (long long)blockIdx.x * kScanThreads + threadIdx.x;
@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(kScanThreads) k_flag_count(long long n, const 
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_flag_compact(long long n, const uint8_t* __restrict__ flag,
-                                                               const int* __restrict__ bcount, int* __restrict__ map,
-                                                               int* __restrict__ list, int cap, int* __restrict__ count) {
+                                                               const int* __restrict__ bcount, int* __restrict__ list,
+                                                               int cap, int* __restrict__ count) {
     __shared__ int s_w[kScanThreads / 32];
     __shared__ int s_base;
     const int t = threadIdx.x, w = t >> 5, l = t & 31;
@@ -190,10 +190,7 @@ __global__ void __launch_bounds__(kScanThreads) k_flag_compact(long long n, cons
     int before = 0;
     for (int q = 0; q < w; q++) before += s_w[q];
     const int r = s_base + before + __popc(m & ((1u << l) - 1u));
-    if (i < n) {
-        map[i] = f ? r : -1;
-        if (f && r < cap) list[r] = (int)i;
-    }
+    if (i < n && list && f && r < cap) list[r] = (int)i;
     if (blockIdx.x == gridDim.x - 1 && t == kScanThreads - 1) {
         int tot = 0;
         for (int q = 0; q < kScanThreads / 32; q++) tot += s_w[q];
@@ -201,12 +198,11 @@ __global__ void __launch_bounds__(kScanThreads) k_flag_compact(long long n, cons
     }
 }
 
-static int flag_compact(long long n, const uint8_t* flag, int* bcount, int* map, int* list, int cap, int* count,
-                        cudaStream_t st) {
+static int flag_compact(long long n, const uint8_t* flag, int* bcount, int* list, int cap, int* count, cudaStream_t st) {
     const unsigned nb = (unsigned)((n + kScanThreads - 1) / kScanThreads);
     pf::count_launch(2);
     k_flag_count<<<nb, kScanThreads, 0, st>>>(n, flag, bcount);
-    k_flag_compact<<<nb, kScanThreads, 0, st>>>(n, flag, bcount, map, list, cap, count);
+    k_flag_compact<<<nb, kScanThreads, 0, st>>>(n, flag, bcount, list, cap, count);
     PF_LAUNCH_CHECK("flag compaction launch");
     return PF_OK;
 }
@@ -214,8 +210,7 @@ static int flag_compact(long long n, const uint8_t* flag, int* bcount, int* map,
 // Ehat of every coarse element, element-major Eh[e * 8 + k] (one 32-byte (FP32) or 64-byte
 // (FP64) run per element, read with vector loads)
 template <typename T>
-__global__ void k_coarse_ehat(int NXc, int NYc, int NZc, const double* __restrict__ E, const int* __restrict__ dmap,
-                              T* __restrict__ Eh) {
+__global__ void k_coarse_ehat(int NXc, int NYc, int NZc, const double* __restrict__ E, T* __restrict__ Eh) {
     const long long ne = (long long)NXc * NYc * NZc;
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= ne) return;
@@ -237,180 +232,39 @@ __global__ void k_coarse_ehat(int NXc, int NYc, int NZc, const double* __restric
                 c[q] = lo + hi;
                 c[q | b] = lo - hi;
             }
-    const int d = dmap ? dmap[e] : -1;
-    if (d >= 0) c[0] = -(double)d - 1.0;
 #pragma unroll
     for (int q = 0; q < 8; q++) Eh[e * 8 + q] = (T)c[q];
 }
 
-template <int DIM>
-struct GridC {
-    int nel[3], nn[3];
-};
-
-__device__ __forceinline__ long long fnode(const GridC<3>& g, int i, int j, int k) {
-    return (long long)k + (long long)g.nn[2] * (i + (long long)g.nn[0] * j);
-}
-__device__ __forceinline__ double hp(int d) { return d == 0 ? 1.0 : d == 1 ? 0.5 : d == 2 ? 0.25 : 0.125; }
-
-// Dirty matrices in the physical basis: thread (d, LI, LJ) writes the 3x3 block of corners
-// LI, LJ of dirty element dlist[d]: the dirty part of A^[I, J] if this element is the first
-// dirty element containing I and J, else 0.  The dirty part: every dirty element containing
-// I and J contributes sum_c E_c (Z Phat_c)^T K0 (Z Phat_c) (children with their fine
-// constraints masked, as the reference's level-0 Galerkin, mgm.cu:247-447); the identity
-// rows are k_ident_rows'.
-__global__ void __launch_bounds__(64) k_dirty_blocks(GridC<3> gf, GridC<3> gc, const double* __restrict__ E,
-                                                     const uint8_t* __restrict__ mask,
-                                                     const uint8_t* __restrict__ elem_flag,
-                                                     const int* __restrict__ dlist, int nd,
-                                                     const double* __restrict__ K0, double* __restrict__ M) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)nd * 64) return;
-    const int d = (int)(t >> 6), LI = (int)((t >> 3) & 7), LJ = (int)(t & 7);
-    const int e = dlist[d];
-    const int NYc = gc.nel[1], NZc = gc.nel[2];
-    const int ez = e % NZc, ey = (e / NZc) % NYc, ex = e / (NZc * NYc);
-    const int I[3] = {ex + kCXd(LI), ey + kCYd(LI), ez + kCZd(LI)};
-    const int J[3] = {ex + kCXd(LJ), ey + kCYd(LJ), ez + kCZd(LJ)};
-    // candidate elements containing I and J: per axis lower corner in [lo_a, hi_a]
-    int lo[3], hi[3];
-    for (int a = 0; a < 3; a++) {
-        const int o = J[a] - I[a];
-        if (o == 0) {
-            lo[a] = I[a] - 1 < 0 ? 0 : I[a] - 1;
-            hi[a] = I[a] > gc.nel[a] - 1 ? gc.nel[a] - 1 : I[a];
-        } else {
-            lo[a] = hi[a] = o > 0 ? I[a] : J[a];
-        }
+// coarse nodes that are corners of a dirty element
+__global__ void k_corner_flags(int NXc, int NYc, int NZc, const uint8_t* __restrict__ elem_flag,
+                               uint8_t* __restrict__ nflag) {
+    const int nx = NXc + 1, nz = NZc + 1;
+    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= (long long)nx * (NYc + 1) * nz) return;
+    const unsigned t = (unsigned)n / nz;
+    const int k = (int)((unsigned)n - t * nz), j = (int)(t / nx), i = (int)(t - (unsigned)j * nx);
+    uint8_t f = 0;
+    for (int q = 0; q < 8; q++) {
+        const int ex = i - kCXd(q), ey = j - kCYd(q), ez = k - kCZd(q);
+        if (ex >= 0 && ey >= 0 && ez >= 0 && ex < NXc && ey < NYc && ez < NZc)
+            f |= elem_flag[((long long)ex * NYc + ey) * NZc + ez];
     }
-    // owner: the first dirty candidate in element order
-    bool owner = false, found = false;
-    for (int cx = lo[0]; cx <= hi[0] && !found; cx++)
-        for (int cy = lo[1]; cy <= hi[1] && !found; cy++)
-            for (int cz = lo[2]; cz <= hi[2] && !found; cz++) {
-                const int ce = (cx * NYc + cy) * NZc + cz;
-                if (elem_flag[ce]) {
-                    owner = ce == e;
-                    found = true;
-                }
-            }
-    double blk[9];
-    for (int q = 0; q < 9; q++) blk[q] = 0.0;
-    if (owner) {
-        for (int cx = lo[0]; cx <= hi[0]; cx++)
-            for (int cy = lo[1]; cy <= hi[1]; cy++)
-                for (int cz = lo[2]; cz <= hi[2]; cz++) {
-                    const int ce = (cx * NYc + cy) * NZc + cz;
-                    if (!elem_flag[ce]) continue;
-                    // local corners of I and J in element (cx, cy, cz)
-                    int li = 0, lj = 0;
-                    for (int q = 0; q < 8; q++) {
-                        if (cx + kCXd(q) == I[0] && cy + kCYd(q) == I[1] && cz + kCZd(q) == I[2]) li = q;
-                        if (cx + kCXd(q) == J[0] && cy + kCYd(q) == J[1] && cz + kCZd(q) == J[2]) lj = q;
-                    }
-                    for (int c = 0; c < 8; c++) {
-                        const int fx = 2 * cx + kCXd(c), fy = 2 * cy + kCYd(c), fz = 2 * cz + kCZd(c);
-                        const double we = E[((long long)fx * gf.nel[1] + fy) * gf.nel[2] + fz];
-                        for (int l = 0; l < 8; l++) {
-                            const int nxl = kCXd(c) + kCXd(l), nyl = kCYd(c) + kCYd(l), nzl = kCZd(c) + kCZd(l);
-                            const double pl = (1.0 - 0.5 * abs(nxl - 2 * kCXd(li))) *
-                                              (1.0 - 0.5 * abs(nyl - 2 * kCYd(li))) *
-                                              (1.0 - 0.5 * abs(nzl - 2 * kCZd(li)));
-                            if (pl == 0.0) continue;
-                            const uint8_t ml = mask[fnode(gf, 2 * cx + nxl, 2 * cy + nyl, 2 * cz + nzl)];
-                            for (int l2 = 0; l2 < 8; l2++) {
-                                const int nx2 = kCXd(c) + kCXd(l2), ny2 = kCYd(c) + kCYd(l2), nz2 = kCZd(c) + kCZd(l2);
-                                const double p2 = (1.0 - 0.5 * abs(nx2 - 2 * kCXd(lj))) *
-                                                  (1.0 - 0.5 * abs(ny2 - 2 * kCYd(lj))) *
-                                                  (1.0 - 0.5 * abs(nz2 - 2 * kCZd(lj)));
-                                if (p2 == 0.0) continue;
-                                const uint8_t m2 = mask[fnode(gf, 2 * cx + nx2, 2 * cy + ny2, 2 * cz + nz2)];
-                                const double f = we * pl * p2;
-                                for (int a = 0; a < 3; a++) {
-                                    if (ml & (1 << a)) continue;
-                                    for (int b = 0; b < 3; b++) {
-                                        if (m2 & (1 << b)) continue;
-                                        blk[a * 3 + b] += f * K0[(l * 3 + a) * 24 + l2 * 3 + b];
-                                    }
-                                }
-                            }
-                        }
-                    }
-                }
-    }
-    double* Md = M + (long long)d * 576;
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) Md[(LI * 3 + a) * 24 + LJ * 3 + b] = blk[a * 3 + b];
+    nflag[n] = f;
 }
 
-// Identity rows of the level-1 Galerkin operator, Phat^T (I - Z) Phat: thread (q, o) writes,
-// for identity node n = nlist[q] and neighbour m = n + o (o = dx + 3 dy + 9 dz + 13), the
-// three per-component coefficients S[(a * 27 + o) * icap + q] = sum over the fine nodes f
-// within one fine spacing of both 2n and 2m whose DOF a is constrained of
-// 0.5^|f - 2n|_0 0.5^|f - 2m|_0 (the interpolation weights; mgm.cu:247-447 adds these rows).
+// S[q * 243 + e] = stencil entry e (neighbour, row, column component) of node nlist[q]
 template <typename T>
-__global__ void k_ident_rows(GridC<3> gf, GridC<3> gc, const uint8_t* __restrict__ mask, const int* __restrict__ nlist,
-                             int nq, int icap, T* __restrict__ S) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)nq * 27) return;
-    const int q = (int)(t / 27), o = (int)(t % 27);
-    const int dx = o % 3 - 1, dy = (o / 3) % 3 - 1, dz = o / 9 - 1;
-    const long long n = nlist[q];
-    const int nk = (int)(n % gc.nn[2]), ni = (int)((n / gc.nn[2]) % gc.nn[0]);
-    const int nj = (int)(n / ((long long)gc.nn[2] * gc.nn[0]));
-    const int mi = ni + dx, mj = nj + dy, mk = nk + dz;
-    double acc[3] = {0.0, 0.0, 0.0};
-    if (mi >= 0 && mj >= 0 && mk >= 0 && mi < gc.nn[0] && mj < gc.nn[1] && mk < gc.nn[2]) {
-        for (int di = -1; di <= 1; di++)
-            for (int dj = -1; dj <= 1; dj++)
-                for (int dk = -1; dk <= 1; dk++) {
-                    const int fi = 2 * ni + di, fj = 2 * nj + dj, fk = 2 * nk + dk;
-                    if (fi < 0 || fj < 0 || fk < 0 || fi >= gf.nn[0] || fj >= gf.nn[1] || fk >= gf.nn[2]) continue;
-                    const int ei = fi - 2 * mi, ej = fj - 2 * mj, ek = fk - 2 * mk;
-                    if (ei < -1 || ei > 1 || ej < -1 || ej > 1 || ek < -1 || ek > 1) continue;
-                    const uint8_t m = mask[fnode(gf, fi, fj, fk)];
-                    if (!m) continue;
-                    const double w = hp((di != 0) + (dj != 0) + (dk != 0)) * hp((ei != 0) + (ej != 0) + (ek != 0));
-                    for (int a = 0; a < 3; a++)
-                        if (m & (1 << a)) acc[a] += w;
-                }
-    }
-    for (int a = 0; a < 3; a++) S[(long long)(a * 27 + o) * icap + q] = (T)acc[a];
-}
-
-// Walsh basis: W = T M T^T / 64, stored Wd[(i * 24 + j) * cap + d] (coalesced across the
-// dirty elements of a warp)
-template <typename T>
-__global__ void __launch_bounds__(576) k_dirty_walsh(const double* __restrict__ M, int cap, T* __restrict__ Wd) {
-    __shared__ double s_m[576], s_u[576];
-    const int d = blockIdx.x, t = threadIdx.x;
-    s_m[t] = M[(long long)d * 576 + t];
+__global__ void __launch_bounds__(256) k_flag_rows(long long N, const double* __restrict__ A, const int* __restrict__ nlist,
+                                                   int nq, T* __restrict__ S) {
+    // threads along q: reads of consecutive nodes coalesce; written through shared memory
+    __shared__ T s_v[27][33];
+    const int q0 = blockIdx.x * 32, l = threadIdx.x & 31, w = threadIdx.x >> 5, e0 = blockIdx.y * 27;
+    const long long n = q0 + l < nq ? nlist[q0 + l] : -1;
+    for (int e = w; e < 27; e += 8) s_v[e][l] = n >= 0 ? (T)A[(long long)(e0 + e) * N + n] : T(0);
     __syncthreads();
-    {  // U = M T^T: U[l][j] = sum_n M[l][(n, a_j)] walsh(m_j, n)
-        const int l = t / 24, j = t % 24, mj = j / 3, aj = j % 3;
-        double s = 0.0;
-        for (int n = 0; n < 8; n++) {
-            int w = 1;
-            const int pos[3] = {kCXd(n), kCYd(n), kCZd(n)};
-            for (int a = 0; a < 3; a++)
-                if ((mj >> a) & 1) w *= pos[a] ? 1 : -1;
-            s += w * s_m[l * 24 + n * 3 + aj];
-        }
-        s_u[t] = s;
-    }
-    __syncthreads();
-    {  // W[i][j] = sum_n walsh(m_i, n) U[(n, a_i)][j] / 64
-        const int i = t / 24, j = t % 24, mi = i / 3, ai = i % 3;
-        double s = 0.0;
-        for (int n = 0; n < 8; n++) {
-            int w = 1;
-            const int pos[3] = {kCXd(n), kCYd(n), kCZd(n)};
-            for (int a = 0; a < 3; a++)
-                if ((mi >> a) & 1) w *= pos[a] ? 1 : -1;
-            s += w * s_u[(n * 3 + ai) * 24 + j];
-        }
-        Wd[(long long)t * cap + d] = (T)(s / 64.0);
-    }
+    for (int q = w; q < 32; q += 8)
+        if (q0 + q < nq && l < 27) S[(long long)(q0 + q) * 243 + e0 + l] = s_v[l][q];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -423,14 +277,11 @@ __device__ __forceinline__ T inv_tw(int n, int nn) {
 }
 
 // Element operator in the Walsh basis.  glo / ghi: transformed lower / upper faces; eh: the
-// element's Ehat (eh[0] < 0 marks a dirty element, index -eh[0] - 1, if the dirty list
-// confirms it for element e).  G receives the lower-face outputs plus the carry of the
-// previous element; carry the upper-face outputs.
+// element's Ehat.  G receives the lower-face outputs plus the carry of the previous element;
+// carry the upper-face outputs.
 template <typename T>
 __device__ __forceinline__ void coarse_element(const T (&glo)[3][2][2], const T (&ghi)[3][2][2], const T (&eh)[8],
-                                               int e, const CoarseCoef<T>& cf, const T* __restrict__ Wd,
-                                               const int* __restrict__ dlist, int cap, T (&carry)[3][2][2],
-                                               T (&G)[3][2][2]) {
+                                               const CoarseCoef<T>& cf, T (&carry)[3][2][2], T (&G)[3][2][2]) {
     T v[24];
 #pragma unroll
     for (int a = 0; a < 3; a++)
@@ -441,36 +292,7 @@ __device__ __forceinline__ void coarse_element(const T (&glo)[3][2][2], const T 
                 v[((0 | (ym << 1) | (zm << 2)) * 3) + a] = ghi[a][ym][zm] + glo[a][ym][zm];
                 v[((1 | (ym << 1) | (zm << 2)) * 3) + a] = ghi[a][ym][zm] - glo[a][ym][zm];
             }
-    // a negative Ehat_0 is a dirty marker only if the dirty list confirms it (densities that
-    // are themselves negative can make Ehat_0 < 0 on a clean element)
-    int d = 0;
-    bool dirty = false;
-    if (eh[0] < T(0) && cap > 0) {
-        const T md = -eh[0] - T(1);
-        if (md >= T(0) && md < T(cap)) {
-            d = (int)md;
-            dirty = dlist[d] == e;
-        }
-    }
-    // outputs slot by slot (component a, y-mode, z-mode; x-modes 0 and 1), folded into G.
-    // FP32: one branch per element between the explicit and the structured matrix; FP64
-    // (254 registers) branches per output, which keeps it free of spills
-    if (sizeof(T) == 4 && dirty) {
-        const T* wd = Wd + d;
-        Unroll<12>::run([&](auto S) {
-            constexpr int slot = decltype(S)::value;
-            constexpr int a = slot / 4, ym = (slot >> 1) & 1, zm = slot & 1;
-            constexpr int i0 = (((ym << 1) | (zm << 2)) * 3) + a, i1 = ((1 | (ym << 1) | (zm << 2)) * 3) + a;
-            T z0 = T(0), z1 = T(0);
-#pragma unroll
-            for (int j = 0; j < 24; j++) z0 = fma(wd[(long long)(i0 * 24 + j) * cap], v[j], z0);
-#pragma unroll
-            for (int j = 0; j < 24; j++) z1 = fma(wd[(long long)(i1 * 24 + j) * cap], v[j], z1);
-            G[a][ym][zm] = (z0 - z1) + carry[a][ym][zm];
-            carry[a][ym][zm] = z0 + z1;
-        });
-        return;
-    }
+    // outputs slot by slot (component a, y-mode, z-mode; x-modes 0 and 1), folded into G
     Unroll<12>::run([&](auto S) {
         constexpr int slot = decltype(S)::value;
         constexpr int a = slot / 4, ym = (slot >> 1) & 1, zm = slot & 1;
@@ -479,11 +301,7 @@ __device__ __forceinline__ void coarse_element(const T (&glo)[3][2][2], const T 
             constexpr int xm = decltype(X)::value;
             constexpr int i = ((xm | (ym << 1) | (zm << 2)) * 3) + a;
             T acc = T(0);
-            if (sizeof(T) == 8 && dirty) {
-                const T* w = Wd + (long long)(i * 24) * cap + d;
-#pragma unroll
-                for (int j = 0; j < 24; j++) acc = fma(w[(long long)j * cap], v[j], acc);
-            } else if constexpr (i >= 3) {
+            if constexpr (i >= 3) {
                 Unroll<8>::run([&](auto K) {
                     constexpr int k = decltype(K)::value;
                     constexpr int q = wclass(i) ^ k;
@@ -505,32 +323,14 @@ __device__ __forceinline__ void coarse_element(const T (&glo)[3][2][2], const T 
     });
 }
 
-// identity rows of owned node (x, y, z), index q: sum over its 27 neighbours m of
-// S(a, m) (D u)_m per component a
-template <typename T>
-__device__ __forceinline__ void coarse_ident(int x, int y, int z, int nx, int ny, int nz, int q, int icap,
-                                             const T* __restrict__ S, const T* __restrict__ u, T (&out)[3]) {
-    T acc[3] = {T(0), T(0), T(0)};
-#pragma unroll 1
-    for (int o = 0; o < 27; o++) {
-        const int mx = x + o % 3 - 1, my = y + (o / 3) % 3 - 1, mz = z + o / 9 - 1;
-        if (mx < 0 || my < 0 || mz < 0 || mx >= nx || my >= ny || mz >= nz) continue;
-        const long long m = (long long)mz + (long long)nz * (mx + (long long)nx * my);
-        const T dm = inv_tw<T>(mx, nx) * inv_tw<T>(my, ny) * inv_tw<T>(mz, nz);
-        for (int a = 0; a < 3; a++) acc[a] = fma(S[(long long)(a * 27 + o) * icap + q], u[3 * m + a] * dm, acc[a]);
-    }
-    for (int a = 0; a < 3; a++) out[a] = acc[a];
-}
-
 // RW element rows per warp: lanes are RW segments of L = 32 / RW along z (shuffles of width L),
 // so a z-tile owns L - 2 node columns; RW = 2 wastes fewer lanes when the level's z extent
 // is just above a multiple of 30 (level 1 of a 256x128x128 grid: 65 node columns).
 template <typename T, int NW, int MINB, int MODE, int RW>
 __global__ void __launch_bounds__(NW * 32, MINB)
     k_coarse_matvec(int NX, int NY, int NZ, int CXc, const T* __restrict__ u, const T* __restrict__ Eh,
-                    const T* __restrict__ Wd, const int* __restrict__ dlist, int cap, const CoarseCoef<T> cf,
-                    Epi<T> epi, const uint8_t* __restrict__ nflag, const int* __restrict__ nmap,
-                    const T* __restrict__ S, int icap) {
+                    const CoarseCoef<T> cf, Epi<T> epi, const uint8_t* __restrict__ nflag,
+                    const int* __restrict__ nlist, const int* __restrict__ nlisted, const T* __restrict__ S) {
     pdl_wait();
     pdl_trigger();
     constexpr int L = 32 / RW, NR = NW * RW, TY = NR - 1;  // lanes per row, rows, owned rows
@@ -557,6 +357,31 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     const T s0 = sz * sy0, s1 = sz * sy1;
     const T so = inv_tw<T>(kc + 1, nz) * sy1;  // owned node (je + 1, kc + 1), without x
     const T wgt = epi_omega(epi);
+
+    // rows of the nodes next to constraints, one warp each: lane o < 27 takes neighbour o
+    if (nflag) {
+        const int nq = *nlisted, gl = tid & 31;
+        const int nwarp = gridDim.x * gridDim.y * gridDim.z * NW;
+        for (int q = (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) * NW + (tid >> 5); q < nq; q += nwarp) {
+            const int n = nlist[q];
+            const unsigned tz = (unsigned)n / nz;
+            const int k = (int)((unsigned)n - tz * nz), j = (int)(tz / nx), i = (int)(tz - (unsigned)j * nx);
+            const int mi = i + gl % 3 - 1, mj = j + (gl / 3) % 3 - 1, mk = k + gl / 9 - 1;
+            T acc[3] = {T(0), T(0), T(0)};
+            if (gl < 27 && mi >= 0 && mj >= 0 && mk >= 0 && mi < nx && mj < ny && mk < nz) {
+                const T* um = u + 3 * ((long long)mk + (long long)nz * (mi + (long long)nx * mj));
+                const T* Sq = S + (long long)q * 243 + gl * 9;
+                const T u0 = um[0], u1 = um[1], u2 = um[2];
+#pragma unroll
+                for (int c = 0; c < 3; c++) acc[c] = fma(Sq[3 * c], u0, fma(Sq[3 * c + 1], u1, Sq[3 * c + 2] * u2));
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(FULL, acc[c], o);
+            if (gl < 3) epi.out[3 * n + gl] = epi_apply(epi, 3 * n + gl, gl == 0 ? acc[0] : gl == 1 ? acc[1] : acc[2], wgt);
+        }
+    }
 
     auto load = [&](int p, T (&v)[2][3]) {
         const bool pok = p >= 0 && p < nx;
@@ -616,13 +441,15 @@ __global__ void __launch_bounds__(NW * 32, MINB)
         const int ie = ix0 - 1 + s;
         face(v, gh);
         if (s < CXc) load(ie + 2, v);
-        const bool out_now = owner && s >= 1 && ie < nx;
         const int no = n1 + 1 + nz * ie;
+        bool out_now = owner && s >= 1 && ie < nx;
         T G[3][2][2];
-        coarse_element<T>(gl, gh, eh, e0 + eplane * ie, cf, Wd, dlist, cap, carry, G);
+        coarse_element<T>(gl, gh, eh, cf, carry, G);
         if (s < CXc) eload(ie + 1, eh);
         T pb[3], px[3], pd[3], pa[3];
+        uint8_t nf = 0;
         if (out_now) {
+            if (nflag) nf = nflag[no];
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 if constexpr (need_b) pb[c] = epi.b[3 * no + c];
@@ -641,13 +468,11 @@ __global__ void __launch_bounds__(NW * 32, MINB)
             s_q[s & 1][c][w][l] = up0 + __shfl_down_sync(FULL, lo0, 1, L);
         }
         __syncthreads();
-        if (out_now) {
+        if (out_now && !nf) {
             const T sc = so * inv_tw<T>(ie, nx);
-            T id[3] = {T(0), T(0), T(0)};
-            if (nflag && nflag[no]) coarse_ident<T>(ie, je + 1, kc + 1, nx, ny, nz, nmap[no], icap, S, u, id);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                const T y = (P1[c] + s_q[s & 1][c][w + 1][l] + id[c]) * sc;
+                const T y = (P1[c] + s_q[s & 1][c][w + 1][l]) * sc;
                 T o = y;
                 if constexpr (MODE == PF_EPI_RESID) {
                     o = pb[c] - y;
@@ -739,10 +564,10 @@ template <typename T, int MODE, int RW>
 static int coarse_launch(dim3 grid, int cx, const Grid& g, const T* u, const CoarseOp* c, const CoarseCoef<T>& cf,
                          const Epi<T>& epi, cudaStream_t st) {
     constexpr int NW = CoarseShape<T>::NW, MINB = CoarseShape<T>::MINB;
-    const uint8_t* nflag = c->nident > 0 ? c->nflag : nullptr;
+    const uint8_t* nflag = c->nrows > 0 ? c->nflag : nullptr;
     PF_CUDA(launch_pdl(k_coarse_matvec<T, NW, MINB, MODE, RW>, grid, dim3(NW * 32), 0, st, g.nel[0], g.nel[1],
-                       g.nel[2], cx, u, (const T*)c->Eh, (const T*)c->Wd, (const int*)c->dlist, c->cap, cf, epi,
-                       nflag, (const int*)c->nmap, (const T*)c->S, c->icap));
+                       g.nel[2], cx, u, (const T*)c->Eh, cf, epi, nflag, (const int*)c->nlist,
+                       (const int*)(c->count + 1), (const T*)c->S));
     return PF_OK;
 }
 
@@ -802,8 +627,7 @@ int coarse_create(const Op* op, int fp32, CoarseOp** out) {
     c->tsize = fp32 ? 4 : 8;
     const long long ne = c->g.n_elem;
     s = calloc_dev(&c->Eh, (size_t)ne * 8 * c->tsize);
-    s = s ? s : calloc_dev((void**)&c->dmap, (size_t)ne * sizeof(int));
-    s = s ? s : calloc_dev((void**)&c->nmap, (size_t)c->g.n_nodes * sizeof(int));
+    s = s ? s : calloc_dev((void**)&c->nflag, (size_t)c->g.n_nodes);
     s = s ? s : calloc_dev((void**)&c->count, 2 * sizeof(int));
     {
         const long long nmax = ne > c->g.n_nodes ? ne : c->g.n_nodes;
@@ -820,109 +644,66 @@ int coarse_create(const Op* op, int fp32, CoarseOp** out) {
 
 void coarse_destroy(CoarseOp* c) {
     if (!c) return;
-    for (void* p : {c->Eh, (void*)c->dmap, (void*)c->dlist, (void*)c->M, c->Wd, (void*)c->count, (void*)c->nmap,
-                    (void*)c->nlist, c->S, (void*)c->bcount})
+    for (void* p : {c->Eh, (void*)c->count, (void*)c->nflag, (void*)c->nlist, c->S, (void*)c->bcount})
         if (p) cudaFree(p);
     if (c->h_count) cudaFreeHost(c->h_count);
     delete c;
 }
 
-static GridC<3> gridc(const Grid& g) {
-    GridC<3> r;
-    for (int a = 0; a < 3; a++) {
-        r.nel[a] = g.nel[a];
-        r.nn[a] = g.nn[a];
-    }
-    return r;
-}
-
-// Ehat and the dirty matrices for densities E (FP64) and the fine node mask.  The dirty
-// list is recounted on every call; the host waits for the count (one int) and grows the
-// dirty storage when it no longer fits.
-int coarse_setup(CoarseOp* c, const double* E, const uint8_t* mask, const uint8_t* elem_flag,
-                 const uint8_t* node_flag, const double* K0_dev, cudaStream_t st, bool* realloc) {
+// Ehat for densities E (FP64), and the assembled rows (level-1 stencil A64) of the nodes next to
+// constraints.  These are recounted on every call; the host waits for the counts (two ints) and
+// grows the rows' storage when they no longer fit.
+int coarse_setup(CoarseOp* c, const double* E, const uint8_t* mask, const uint8_t* elem_flag, const double* A64,
+                 cudaStream_t st, bool* realloc) {
     *realloc = false;
     const Grid& gc = c->g;
     const long long ne = gc.n_elem;
     if (ne >= (1LL << 31) || gc.n_nodes >= (1LL << 31)) return fail(PF_BAD_ARG, "coarse grid too large");
     int nd = 0, ni = 0;
-    c->nflag = node_flag;
     if (mask) {
+        pf::count_launch();
+        k_corner_flags<<<(unsigned)((gc.n_nodes + 255) / 256), 256, 0, st>>>(gc.nel[0], gc.nel[1], gc.nel[2], elem_flag,
+                                                                           c->nflag);
         for (int pass = 0; pass < 2; pass++) {
-            int s = flag_compact(ne, elem_flag, c->bcount, c->dmap, c->dlist, c->cap, c->count, st);
-            s = s ? s : flag_compact(gc.n_nodes, node_flag, c->bcount, c->nmap, c->nlist, c->icap, c->count + 1, st);
+            int s = pass ? (int)PF_OK : flag_compact(ne, elem_flag, c->bcount, nullptr, 0, c->count, st);
+            s = s ? s : flag_compact(gc.n_nodes, c->nflag, c->bcount, c->nlist, c->cap, c->count + 1, st);
             if (s) return s;
             PF_CUDA(cudaMemcpyAsync(c->h_count, c->count, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
             PF_CUDA(cudaStreamSynchronize(st));
             nd = c->h_count[0];
             ni = c->h_count[1];
-            if (nd <= c->cap && ni <= c->icap) break;
             if (nd >= (1 << 24)) return fail(PF_UNSUPPORTED, "coarse operator: %d dirty elements (limit 2^24)", nd);
-            if (nd > c->cap) {
-                for (void* p : {(void*)c->dlist, (void*)c->M, c->Wd})
-                    if (p) cudaFree(p);
-                c->dlist = nullptr;
-                c->M = nullptr;
-                c->Wd = nullptr;
-                const int cap = nd + nd / 4 + 32;
-                int s = calloc_dev((void**)&c->dlist, (size_t)cap * sizeof(int));
-                s = s ? s : calloc_dev((void**)&c->M, (size_t)cap * 576 * sizeof(double));
-                s = s ? s : calloc_dev(&c->Wd, (size_t)cap * 576 * c->tsize);
-                if (s) {
-                    c->cap = 0;
-                    return s;
-                }
-                c->cap = cap;
-            }
-            if (ni > c->icap) {
-                for (void* p : {(void*)c->nlist, c->S})
-                    if (p) cudaFree(p);
-                c->nlist = nullptr;
-                c->S = nullptr;
-                const int icap = ni + ni / 4 + 32;
-                int s = calloc_dev((void**)&c->nlist, (size_t)icap * sizeof(int));
-                s = s ? s : calloc_dev(&c->S, (size_t)icap * 81 * c->tsize);
-                if (s) {
-                    c->icap = 0;
-                    return s;
-                }
-                c->icap = icap;
-            }
+            if (ni <= c->cap) break;
+            for (void* p : {(void*)c->nlist, c->S})
+                if (p) cudaFree(p);
+            c->nlist = nullptr;
+            c->S = nullptr;
+            c->cap = 0;
+            const int cap = ni + ni / 4 + 32;
+            s = calloc_dev((void**)&c->nlist, (size_t)cap * sizeof(int));
+            s = s ? s : calloc_dev(&c->S, (size_t)cap * 243 * c->tsize);
+            if (s) return s;
+            c->cap = cap;
             *realloc = true;
         }
     }
-    c->nident = ni;
+    c->nrows = ni;
     c->ndirty = nd;
     const unsigned nb = (unsigned)((ne + 255) / 256);
     pf::count_launch();
     if (c->tsize == 4)
-        k_coarse_ehat<float><<<nb, 256, 0, st>>>(gc.nel[0], gc.nel[1], gc.nel[2], E, mask ? c->dmap : nullptr,
-                                                 (float*)c->Eh);
+        k_coarse_ehat<float><<<nb, 256, 0, st>>>(gc.nel[0], gc.nel[1], gc.nel[2], E, (float*)c->Eh);
     else
-        k_coarse_ehat<double><<<nb, 256, 0, st>>>(gc.nel[0], gc.nel[1], gc.nel[2], E, mask ? c->dmap : nullptr,
-                                                  (double*)c->Eh);
+        k_coarse_ehat<double><<<nb, 256, 0, st>>>(gc.nel[0], gc.nel[1], gc.nel[2], E, (double*)c->Eh);
     PF_LAUNCH_CHECK("coarse ehat launch");
-    if (nd > 0) {
-        pf::count_launch(2);
-        k_dirty_blocks<<<(unsigned)(((long long)nd * 64 + 63) / 64), 64, 0, st>>>(
-            gridc(c->fine), gridc(gc), E, mask, elem_flag, c->dlist, nd, K0_dev, c->M);
-        PF_LAUNCH_CHECK("dirty blocks launch");
-        if (c->tsize == 4)
-            k_dirty_walsh<float><<<nd, 576, 0, st>>>(c->M, c->cap, (float*)c->Wd);
-        else
-            k_dirty_walsh<double><<<nd, 576, 0, st>>>(c->M, c->cap, (double*)c->Wd);
-        PF_LAUNCH_CHECK("dirty walsh launch");
-    }
     if (ni > 0) {
         pf::count_launch();
-        const unsigned nbi = (unsigned)(((long long)ni * 27 + 255) / 256);
+        const dim3 gr((unsigned)((ni + 31) / 32), 9);
         if (c->tsize == 4)
-            k_ident_rows<float><<<nbi, 256, 0, st>>>(gridc(c->fine), gridc(gc), mask, c->nlist, ni, c->icap,
-                                                     (float*)c->S);
+            k_flag_rows<float><<<gr, 256, 0, st>>>(gc.n_nodes, A64, c->nlist, ni, (float*)c->S);
         else
-            k_ident_rows<double><<<nbi, 256, 0, st>>>(gridc(c->fine), gridc(gc), mask, c->nlist, ni, c->icap,
-                                                      (double*)c->S);
-        PF_LAUNCH_CHECK("identity rows launch");
+            k_flag_rows<double><<<gr, 256, 0, st>>>(gc.n_nodes, A64, c->nlist, ni, (double*)c->S);
+        PF_LAUNCH_CHECK("constrained rows launch");
     }
     return PF_OK;
 }
