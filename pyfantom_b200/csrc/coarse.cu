@@ -336,7 +336,8 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     constexpr int L = 32 / RW, NR = NW * RW, TY = NR - 1;  // lanes per row, rows, owned rows
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ T s_q[2][3][NR][L];
-    if (epi.skip && *epi.skip) return;
+    const int nq = nflag ? *nlisted : 0, done = epi.skip ? *epi.skip : 0;
+    if (done) return;
     constexpr bool need_b = MODE != PF_EPI_STORE, need_x = MODE == PF_EPI_JACOBI || MODE == PF_EPI_JACOBI_ADD;
     constexpr bool need_xa = MODE == PF_EPI_JACOBI_ADD;
     const int nx = NX + 1, ny = NY + 1, nz = NZ + 1;
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
 
     // rows of the nodes next to constraints, one warp each: lane o < 27 takes neighbour o
     if (nflag) {
-        const int nq = *nlisted, gl = tid & 31;
+        const int gl = tid & 31;
         const int nwarp = gridDim.x * gridDim.y * gridDim.z * NW;
         for (int q = (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) * NW + (tid >> 5); q < nq; q += nwarp) {
             const int n = nlist[q];

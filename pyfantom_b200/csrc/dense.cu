@@ -150,12 +150,14 @@ __global__ void __launch_bounds__(256) k_dense_matvec(const double* __restrict__
                                                       const T* __restrict__ b, T* __restrict__ x, const int* skip) {
     pdl_wait();
     pdl_trigger();
-    if (skip && *skip) return;
+    const int done = skip ? *skip : 0;
     const int row = blockIdx.x * 8 + (threadIdx.x >> 5), l = threadIdx.x & 31;
     if (row >= n) return;
     const double* Ar = Ainv + (long long)row * np;
     double s = 0.0;
+#pragma unroll 8
     for (int c = l; c < n; c += 32) s += Ar[c] * (double)b[c];
+    if (done) return;
     s = warp_sum(s);
     if (l == 0) x[row] = (T)s;
 }

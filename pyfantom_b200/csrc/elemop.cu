@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     __shared__ T s_q[2][3][NW * 32];  // [w * L + l]
     __shared__ double s_red[NW];
     __shared__ T s_blk[72];
-    if (epi.skip && *epi.skip) return;
+    const int done = epi.skip ? *epi.skip : 0;  // looked at once the first plane is on its way
     constexpr int mode = MODE;
     constexpr bool need_b = mode != PF_EPI_STORE, need_x = mode == PF_EPI_JACOBI || mode == PF_EPI_JACOBI_ADD;
     constexpr bool need_xa = mode == PF_EPI_JACOBI_ADD;
@@ -532,6 +532,8 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     T vA[2][3];
     int mA0, mA1;
     load(ix0 - 1, vA, mA0, mA1);
+    T eA = escale(ix0 - 1);
+    if (done) return;
     face(vA, mA0, mA1, gA);
     load(ix0, vA, mA0, mA1);
 #pragma unroll
@@ -540,7 +542,6 @@ __global__ void __launch_bounds__(NW * 32, MINB)
         for (int a = 0; a < 2; a++)
 #pragma unroll
             for (int b = 0; b < 2; b++) carry[c][a][b] = T(0);
-    T eA = escale(ix0 - 1);
     for (int s = 0; s <= CXc; s++) {
         step(s, gA, gB, vA, mA0, mA1, eA);
         // the upper face becomes the next lower face (computed values: no wait)

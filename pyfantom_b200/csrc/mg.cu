@@ -36,8 +36,18 @@ struct PcgState {
     double rho_old, norm_b, alpha, beta, R, omega;
     double tol, min_omega, d_omega;
     int it, maxiter, done, status;
-    int stop_le;  // 1: stop when R <= tol (cupyx cg, plain CG); 0: R < tol (MultiGrid)
+    int stop_le;     // 1: stop when R <= tol (cupyx cg, plain CG); 0: R < tol (MultiGrid)
+    int xlag;        // 1: the last iteration's x += alpha p is still to come
     double coef[3];  // deflation: G^-1 Q^T r (start) or G^-1 W^T z (iterations)
+};
+
+enum PcgStep {
+    PCG_NORMB = 1,       // sum = b.b: start of a solve
+    PCG_ALPHA = 2,       // sum = p.q
+    PCG_CHECK = 3,       // sum = r.r: residual, stopping test, Jacobi weight
+    PCG_CHECK_BETA = 4,  // the same, then PCG_BETA (plain CG, z = r)
+    PCG_RHO0 = 5,        // sum = r.z of the start
+    PCG_BETA = 6         // sum = r.z
 };
 
 struct Level {
@@ -154,104 +164,50 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_partial(long long n, const 
 
 __device__ double sum_partials(const double* partials, long long np, double* s_red) {
     double s = 0.0;
-    for (long long i = threadIdx.x; i < np; i += blockDim.x) s += partials[i];
+#pragma unroll 4
+    for (long long i = threadIdx.x; i < np; i += kRedThreads) s += partials[i];
     return block_sum<kRedThreads>(s, s_red);
 }
 
 __device__ void defl_coef(const double* partials, long long np, int off, const double* dG, PcgState* st,
                           double* s_red);
 
-__global__ void __launch_bounds__(kRedThreads) k_pcg_normb(const double* partials, long long np, PcgState* st) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ double s_red[kRedThreads / 32];
-    const double bb = sum_partials(partials, np, s_red);
-    if (threadIdx.x == 0) {
-        st->norm_b = sqrt(bb);
+// the scalar steps between the vector kernels
+// by one thread
+__device__ __forceinline__ void pcg_step(int step, double s, PcgState* st) {
+    if (step == PCG_NORMB) {
+        st->norm_b = sqrt(s);
         st->it = 0;
         st->done = 0;
         st->status = PF_NOT_CONVERGED;
         st->R = 0.0;
         st->omega = st->min_omega;
-        if (!(bb == bb) || isinf(bb)) {
+        if (!(s == s) || isinf(s)) {
             st->done = 1;
             st->status = PF_NONFINITE;
-        } else if (bb == 0.0) {
+        } else if (s == 0.0) {
             st->done = 1;
             st->status = PF_OK;
         }
+        return;
     }
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_pcg_rho0(const double* partials, long long np, PcgState* st,
-                                                          const double* dG) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ double s_red[kRedThreads / 32];
-    if (st->done) return;
-    const double rz = sum_partials(partials, np, s_red);
-    if (dG) defl_coef(partials, np, 1, dG, st, s_red);  // G^-1 W^T z
-    if (threadIdx.x == 0) {
-        st->rho_old = rz;
-        if (!isfinite(rz)) {
+    if (step == PCG_ALPHA) {
+        if (!isfinite(s) || !isfinite(st->rho_old)) {
             st->done = 1;
             st->status = PF_NONFINITE;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_pcg_alpha(const double* partials, long long np, PcgState* st) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ double s_red[kRedThreads / 32];
-    if (st->done) return;
-    const double pq = sum_partials(partials, np, s_red);
-    if (threadIdx.x == 0) {
-        if (!isfinite(pq) || !isfinite(st->rho_old)) {
-            st->done = 1;
-            st->status = PF_NONFINITE;
-        } else if (!(pq > 0.0)) {
+        } else if (!(s > 0.0)) {
             st->done = 1;
             st->status = PF_BREAKDOWN;
         } else {
-            st->alpha = st->rho_old / pq;
+            st->alpha = st->rho_old / s;
         }
+        return;
     }
-}
-
-// x += alpha p, r -= alpha q, partial sums of r.r; with rf (mixed form) also the FP32 copy
-// of r that the V-cycle reads
-__global__ void __launch_bounds__(kRedThreads) k_pcg_xr(long long n, const double* __restrict__ p,
-                                                        const double* __restrict__ q, double* __restrict__ x,
-                                                        double* __restrict__ r, const PcgState* st, double* partials,
-                                                        float* __restrict__ rf) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ double s_red[kRedThreads / 32];
-    if (st->done) return;
-    const double a = st->alpha;
-    double s = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        x[i] += a * p[i];
-        const double ri = r[i] - a * q[i];
-        r[i] = ri;
-        if (rf) rf[i] = (float)ri;
-        s += ri * ri;
-    }
-    s = block_sum<kRedThreads>(s, s_red);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
-}
-
-__global__ void __launch_bounds__(kRedThreads) k_pcg_check(const double* partials, long long np, PcgState* st) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ double s_red[kRedThreads / 32];
-    if (st->done) return;
-    const double rr = sum_partials(partials, np, s_red);
-    if (threadIdx.x == 0) {
-        const double R = sqrt(rr) / st->norm_b;
+    if (step == PCG_CHECK || step == PCG_CHECK_BETA) {
+        const double R = sqrt(s) / st->norm_b;
         st->R = R;
         st->it += 1;
+        st->xlag = 1;
         if (!isfinite(R)) {
             st->done = 1;
             st->status = PF_NONFINITE;
@@ -265,26 +221,55 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_check(const double* partial
             const double c = R < st->tol ? st->tol : (R > 0.1 ? 0.1 : R);
             st->omega = st->min_omega + st->d_omega / 2.0 * exp((-c + st->tol) * 500.0);
         }
+        if (step == PCG_CHECK || st->done) return;
+    }
+    if (!isfinite(s)) {
+        st->done = 1;
+        st->status = PF_NONFINITE;
+        if (step == PCG_RHO0) st->rho_old = s;
+    } else {
+        if (step != PCG_RHO0) st->beta = s / st->rho_old;
+        st->rho_old = s;
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_pcg_beta(const double* partials, long long np, PcgState* st,
+// One block: the sum of the partial sums of the kernel before, and its step.  (Taking the step in
+// the last block of that kernel instead, three launches fewer per iteration, measured 1 % slower
+// at 96x48x48: the fence, the atomic and the reload cost more than a dependent launch.)
+__global__ void __launch_bounds__(kRedThreads) k_pcg_step(const double* partials, long long np, PcgState* st, int step,
                                                           const double* dG) {
     pdl_wait();
     pdl_trigger();
     __shared__ double s_red[kRedThreads / 32];
-    if (st->done) return;
-    const double rz = sum_partials(partials, np, s_red);
-    if (dG) defl_coef(partials, np, 1, dG, st, s_red);  // G^-1 W^T z
-    if (threadIdx.x == 0) {
-        if (!isfinite(rz)) {
-            st->done = 1;
-            st->status = PF_NONFINITE;
-        } else {
-            st->beta = rz / st->rho_old;
-            st->rho_old = rz;
-        }
+    const int done = step != PCG_NORMB && st->done;  // looked at once the partial sums have arrived
+    const double s = sum_partials(partials, np, s_red);
+    if (done) {
+        if (step == PCG_ALPHA && threadIdx.x == 0) st->xlag = 0;  // the iteration after the last: x is complete
+        return;
     }
+    if (dG) defl_coef(partials, np, 1, dG, st, s_red);  // G^-1 W^T z
+    if (threadIdx.x == 0) pcg_step(step, s, st);
+}
+
+// r -= alpha q, partial sums of r.r; with rf (mixed form) also the FP32 copy of r that
+// the V-cycle reads.  x += alpha p follows in k_pcg_p, which reads p anyway.
+__global__ void __launch_bounds__(kRedThreads) k_pcg_r(long long n, const double* __restrict__ q, double* __restrict__ r,
+                                                       const PcgState* st, double* partials, float* __restrict__ rf) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double s_red[kRedThreads / 32];
+    if (st->done) return;
+    const double a = st->alpha;
+    double s = 0.0;
+#pragma unroll 4
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const double ri = r[i] - a * q[i];
+        r[i] = ri;
+        if (rf) rf[i] = (float)ri;
+        s += ri * ri;
+    }
+    s = block_sum<kRedThreads>(s, s_red);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
 }
 
 // component i % dof of a grid-stride loop, advanced without a 64-bit division per element
@@ -298,27 +283,40 @@ struct CompIter {
     }
 };
 
-// p = z + beta p (init: p = z); with the deflation field yf, z - Q coef in place of z
+// x += alpha p, then p = z + beta p (init: p = z alone); with the deflation field yf, z - Q coef
+// in place of z.  After the iteration that ends the solve only x is still to be updated (xlag).
 template <typename TZ>
-__global__ void k_pcg_p(long long n, const TZ* __restrict__ z, double* __restrict__ p, const PcgState* st, int init,
-                        const float* __restrict__ yf, int dof) {
+__global__ void __launch_bounds__(kRedThreads) k_pcg_p(long long n, const TZ* __restrict__ z, double* __restrict__ p,
+                                                       double* __restrict__ x, const PcgState* st, int init,
+                                                       const float* __restrict__ yf, int dof) {
     pdl_wait();
     pdl_trigger();
-    if (st->done) return;
-    const double b = st->beta;
+    const int done = st->done, xlag = init ? 0 : st->xlag;
+    if (done && !xlag) return;
+    const double a = st->alpha, b = st->beta;
     const double c0 = st->coef[0], c1 = st->coef[1], c2 = st->coef[2];
     const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-    if (yf) {
+    if (done) {
+        for (long long i = i0; i < n; i += stride) x[i] += a * p[i];
+    } else if (init) {
+        CompIter ci(i0, stride, dof);
+        for (long long i = i0; i < n; i += stride, ci.next())
+            p[i] = yf ? (double)z[i] - (double)yf[i] * (ci.c == 0 ? c0 : ci.c == 1 ? c1 : c2) : (double)z[i];
+    } else if (yf) {
         CompIter ci(i0, stride, dof);
 #pragma unroll 4
         for (long long i = i0; i < n; i += stride, ci.next()) {
             const double zi = (double)z[i] - (double)yf[i] * (ci.c == 0 ? c0 : ci.c == 1 ? c1 : c2);
-            p[i] = init ? zi : zi + b * p[i];
+            const double pi = p[i];
+            x[i] += a * pi;
+            p[i] = zi + b * pi;
         }
     } else {
+#pragma unroll 4
         for (long long i = i0; i < n; i += stride) {
-            const double zi = (double)z[i];
-            p[i] = init ? zi : zi + b * p[i];
+            const double zi = (double)z[i], pi = p[i];
+            x[i] += a * pi;
+            p[i] = zi + b * pi;
         }
     }
 }
@@ -935,55 +933,59 @@ extern "C" int pf_mg_vcycle(pf_mg* mg, const double* r, double* z, double omega,
     return PF_OK;
 }
 
-// apply the preconditioner to mg->r, leave r.z partials in mg->partials and return z
-// (mixed form: r32_ready = the FP32 copy of r is already in the V-cycle's input)
-static int precondition(pf_mg* mg, const void** z_out, long long* np_out, cudaStream_t st, bool r32_ready) {
+// apply the preconditioner to mg->r and take the PCG step on r.z (PCG_RHO0 or PCG_BETA); z is
+// returned (mixed form: r32_ready = the FP32 copy of r is already in the V-cycle's input)
+static int precondition(pf_mg* mg, const void** z_out, int step, cudaStream_t st, bool r32_ready) {
     const long long n = mg->L[0].ndof;
+    const int* skip = &mg->st->done;
+    long long np = vec_blocks(n);
+    const dim3 vb(vec_blocks(n)), th(kRedThreads);
     int s;
     if (mg->fp32) {
         if (!r32_ready) {
             pf::count_launch();
-            PF_CUDA(launch_pdl(k_d2f_skip, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, mg->r, (float*)mg->L[0].b,
-                               &mg->st->done));
+            PF_CUDA(launch_pdl(k_d2f_skip, vb, th, 0, st, n, mg->r, (float*)mg->L[0].b, &mg->st->done));
         }
         float* res;
         if ((s = vcycle<float>(mg, 0, (const float*)mg->L[0].b, &res, nullptr, nullptr, st))) return s;
         pf::count_launch();
         if (mg->defl)  // r.z and W^T z
-            PF_CUDA(launch_pdl(k_dot_defl<float>, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, (const double*)mg->r,
-                               (const float*)res, (const double*)mg->Wd, mg->partials, (const int*)&mg->st->done));
+            PF_CUDA(launch_pdl(k_dot_defl<float>, vb, th, 0, st, n, (const double*)mg->r, (const float*)res,
+                               (const double*)mg->Wd, mg->partials, skip));
         else
-            PF_CUDA(launch_pdl(k_dot_partial<float>, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, mg->r, res, mg->partials, &mg->st->done));
+            PF_CUDA(launch_pdl(k_dot_partial<float>, vb, th, 0, st, n, mg->r, res, mg->partials, skip));
         PF_LAUNCH_CHECK("dot launch");
         *z_out = res;
-        *np_out = vec_blocks(n);
     } else {
         double* res;
         if (mg->defl) {
             if ((s = vcycle<double>(mg, 0, mg->r, &res, nullptr, nullptr, st))) return s;
             pf::count_launch();
-            PF_CUDA(launch_pdl(k_dot_defl<double>, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, (const double*)mg->r,
-                               (const double*)res, (const double*)mg->Wd, mg->partials, (const int*)&mg->st->done));
+            PF_CUDA(launch_pdl(k_dot_defl<double>, vb, th, 0, st, n, (const double*)mg->r, (const double*)res,
+                               (const double*)mg->Wd, mg->partials, skip));
             PF_LAUNCH_CHECK("dot launch");
-            *np_out = vec_blocks(n);
-        } else {
-            if ((s = vcycle<double>(mg, 0, mg->r, &res, mg->partials, mg->r, st))) return s;
-            *np_out = fine_matvec_num_blocks(mg->op, 0);
+        } else if ((s = vcycle<double>(mg, 0, mg->r, &res, mg->partials, mg->r, st))) {
+            return s;
         }
         *z_out = res;
+        if (!mg->defl) np = fine_matvec_num_blocks(mg->op, 0);
     }
+    pf::count_launch();
+    PF_CUDA(launch_pdl(k_pcg_step, dim3(1), th, 0, st, (const double*)mg->partials, np, mg->st, step,
+                       (const double*)(mg->defl ? mg->dG : nullptr)));
+    PF_LAUNCH_CHECK("pcg step launch");
     return PF_OK;
 }
 
-static int update_p(pf_mg* mg, const void* z, int init, cudaStream_t st) {
+static int update_p(pf_mg* mg, const void* z, double* x, int init, cudaStream_t st) {
     const long long n = mg->L[0].ndof;
+    const dim3 vb(vec_blocks(n)), th(kRedThreads);
+    const float* yf = mg->defl ? mg->yf : nullptr;
     pf::count_launch();
     if (mg->fp32)
-        PF_CUDA(launch_pdl(k_pcg_p<float>, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, (const float*)z, mg->p, mg->st, init,
-                           (const float*)(mg->defl ? mg->yf : nullptr), mg->op->grid.dof));
+        PF_CUDA(launch_pdl(k_pcg_p<float>, vb, th, 0, st, n, (const float*)z, mg->p, x, mg->st, init, yf, mg->op->grid.dof));
     else
-        PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, (const double*)z, mg->p, mg->st, init,
-                           (const float*)(mg->defl ? mg->yf : nullptr), mg->op->grid.dof));
+        PF_CUDA(launch_pdl(k_pcg_p<double>, vb, th, 0, st, n, (const double*)z, mg->p, x, mg->st, init, yf, mg->op->grid.dof));
     PF_LAUNCH_CHECK("p update launch");
     return PF_OK;
 }
@@ -992,28 +994,26 @@ static int pcg_iteration(pf_mg* mg, double* x, cudaStream_t st) {
     const long long n = mg->L[0].ndof;
     const int* skip = &mg->st->done;
     int s;
-    // q = K p, p.q
+    // q = K p, p.q, alpha
     Epi<double> e = make_epi<double>(PF_EPI_STORE, nullptr, nullptr, nullptr, nullptr, mg->q, nullptr, 1.0, skip);
     e.dot_partial = mg->partials;
     e.dot_a = mg->p;
     e.dot_of_y = 1;
     if ((s = fine_mv<double>(mg, mg->p, e, st))) return s;
+    auto take = [&](int step, long long np) {
+        pf::count_launch();
+        return launch_pdl(k_pcg_step, dim3(1), dim3(kRedThreads), 0, st, (const double*)mg->partials, np, mg->st, step,
+                          (const double*)nullptr);
+    };
+    PF_CUDA(take(PCG_ALPHA, fine_matvec_num_blocks(mg->op, 0)));
     pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_alpha, dim3(1), dim3(kRedThreads), 0, st, mg->partials, fine_matvec_num_blocks(mg->op, 0), mg->st));
-    pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_xr, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, mg->p, mg->q, x, mg->r, mg->st, mg->partials,
+    PF_CUDA(launch_pdl(k_pcg_r, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, mg->q, mg->r, mg->st, mg->partials,
                        mg->fp32 ? (float*)mg->L[0].b : (float*)nullptr));
-    pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_check, dim3(1), dim3(kRedThreads), 0, st, mg->partials, vec_blocks(n), mg->st));
+    PF_CUDA(take(PCG_CHECK, vec_blocks(n)));
     PF_LAUNCH_CHECK("pcg launch");
     const void* z;
-    long long np;
-    if ((s = precondition(mg, &z, &np, st, true))) return s;
-    pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_beta, dim3(1), dim3(kRedThreads), 0, st, mg->partials, np, mg->st,
-                       (const double*)(mg->defl ? mg->dG : nullptr)));
-    PF_LAUNCH_CHECK("beta launch");
-    return update_p(mg, z, 0, st);
+    if ((s = precondition(mg, &z, PCG_BETA, st, true))) return s;
+    return update_p(mg, z, x, 0, st);
 }
 
 // Capture the launches `body` issues on the private stream into an executable graph.
@@ -1051,7 +1051,8 @@ static int solve_start(pf_mg* mg, int use_x0, cudaStream_t st) {
     pf::count_launch();
     PF_CUDA(launch_pdl(k_dot_partial<double>, dim3(vec_blocks(n)), dim3(kRedThreads), 0, st, n, mg->bi, mg->bi, mg->partials, nullptr));
     pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_normb, dim3(1), dim3(kRedThreads), 0, st, mg->partials, vec_blocks(n), mg->st));
+    PF_CUDA(launch_pdl(k_pcg_step, dim3(1), dim3(kRedThreads), 0, st, (const double*)mg->partials, (long long)vec_blocks(n),
+                       mg->st, (int)PCG_NORMB, (const double*)nullptr));
     PF_LAUNCH_CHECK("pcg start");
     if (mg->defl) {  // x += Q G^-1 Q^T r, r = b - A x
         const unsigned vb = vec_blocks(n);
@@ -1067,12 +1068,8 @@ static int solve_start(pf_mg* mg, int use_x0, cudaStream_t st) {
         if ((s = fine_mv<double>(mg, mg->xi, e, st))) return s;
     }
     const void* z;
-    long long np;
-    if ((s = precondition(mg, &z, &np, st, false))) return s;
-    pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_rho0, dim3(1), dim3(kRedThreads), 0, st, mg->partials, np, mg->st,
-                       (const double*)(mg->defl ? mg->dG : nullptr)));
-    return update_p(mg, z, 1, st);
+    if ((s = precondition(mg, &z, PCG_RHO0, st, false))) return s;
+    return update_p(mg, z, mg->xi, 1, st);
 }
 
 extern "C" int pf_mg_solve(pf_mg* mg, const double* b, double* x, int use_x0, double tol, int maxiter,
@@ -1211,15 +1208,18 @@ extern "C" int pf_cg_solve(const pf_op* op, const double* E, const uint8_t* node
     }
     const unsigned vb = vec_blocks(n);
     pf::count_launch();
+    auto take = [&](int step, long long np) {
+        pf::count_launch();
+        return launch_pdl(k_pcg_step, dim3(1), dim3(kRedThreads), 0, st, (const double*)partials, np, S, step,
+                          (const double*)nullptr);
+    };
     PF_CUDA(launch_pdl(k_dot_partial<double>, dim3(vb), dim3(kRedThreads), 0, st, n, b, b, partials, nullptr));
-    pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_normb, dim3(1), dim3(kRedThreads), 0, st, partials, vb, S));
+    PF_CUDA(take(PCG_NORMB, vb));
     pf::count_launch();
     PF_CUDA(launch_pdl(k_dot_partial<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, r, partials, skip));
+    PF_CUDA(take(PCG_RHO0, vb));
     pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_rho0, dim3(1), dim3(kRedThreads), 0, st, partials, vb, S, (const double*)nullptr));
-    pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, p, S, 1, (const float*)nullptr, 3));
+    PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, p, x, S, 1, (const float*)nullptr, 3));
     PF_LAUNCH_CHECK("cg start");
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -1227,7 +1227,6 @@ extern "C" int pf_cg_solve(const pf_op* op, const double* E, const uint8_t* node
     cudaEventRecord(e0, st);
     PcgState h;
     int it = 0;
-    const long long nbm = fine_matvec_num_blocks(op, 0);
     while (it < maxiter) {
         const int chunk = (maxiter - it) < 8 ? (maxiter - it) : 8;
         for (int k = 0; k < chunk; k++) {
@@ -1237,16 +1236,12 @@ extern "C" int pf_cg_solve(const pf_op* op, const double* E, const uint8_t* node
             e.dot_of_y = 1;
             int s = launch_fine_matvec<double, double>(op, E, p, node_mask, e, st);
             if (s) return s;
+            PF_CUDA(take(PCG_ALPHA, fine_matvec_num_blocks(op, 0)));
             pf::count_launch();
-            PF_CUDA(launch_pdl(k_pcg_alpha, dim3(1), dim3(kRedThreads), 0, st, partials, nbm, S));
+            PF_CUDA(launch_pdl(k_pcg_r, dim3(vb), dim3(kRedThreads), 0, st, n, q, r, S, partials, (float*)nullptr));
+            PF_CUDA(take(PCG_CHECK_BETA, vb));
             pf::count_launch();
-            PF_CUDA(launch_pdl(k_pcg_xr, dim3(vb), dim3(kRedThreads), 0, st, n, p, q, x, r, S, partials, (float*)nullptr));
-            pf::count_launch();
-            PF_CUDA(launch_pdl(k_pcg_check, dim3(1), dim3(kRedThreads), 0, st, partials, vb, S));
-            pf::count_launch();
-            PF_CUDA(launch_pdl(k_pcg_beta, dim3(1), dim3(kRedThreads), 0, st, partials, vb, S, (const double*)nullptr));
-            pf::count_launch();
-            PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, p, S, 0, (const float*)nullptr, 3));
+            PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, p, x, S, 0, (const float*)nullptr, 3));
         }
         PF_LAUNCH_CHECK("cg iteration");
         it += chunk;

@@ -84,11 +84,13 @@ __global__ void k_restrict(GridDev<DIM> gf, GridDev<DIM> gc, const TI* __restric
     pdl_wait();
     pdl_trigger();
     using TA = TO;  // accumulation precision
-    if (skip && *skip) return;
+    const int done = skip ? *skip : 0;  // looked at only once the values are on their way
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= gc.n_nodes * DIM) return;
     const long long c = (unsigned)t / DIM;
     const int d = (int)(t - c * DIM);
+    TO jw = TO(0);
+    if (j0.x) jw = (TO)((*j0.omega) * j0.scale) * j0.dinv[c * DIM + d];
     int ic, jc, kc;
     ndec(gc, c, ic, jc, kc);
     const int fi = 2 * ic, fj = 2 * jc, fk = 2 * kc;
@@ -97,32 +99,43 @@ __global__ void k_restrict(GridDev<DIM> gf, GridDev<DIM> gc, const TI* __restric
     TA tk = TA(1);
     if (DIM == 3) tk = (kc == 0 || kc == gc.nn[2] - 1) ? TA(1.0 / 1.5) : TA(0.5);
     constexpr int KR = DIM == 3 ? 1 : 0;
+    // values outside the grid are not read but their place in the sums is kept, so that the loads
+    // need no branches and are all in flight together
+    TA v[DIM == 3 ? 27 : 9];
+    const bool ok_i[3] = {fi > 0, true, fi + 1 < gf.nn[0]}, ok_j[3] = {fj > 0, true, fj + 1 < gf.nn[1]};
+    const bool ok_k[3] = {fk > 0, true, fk + 1 < gf.nn[2]};
+    const TI* base = vf + nidx(gf, fi, fj, fk) * DIM + d;
+    const int si = DIM == 3 ? gf.nn[2] * DIM : DIM, sj = si * gf.nn[0];
+#pragma unroll
+    for (int dj = -1; dj <= 1; dj++)
+#pragma unroll
+        for (int di = -1; di <= 1; di++)
+#pragma unroll
+            for (int dk = -KR; dk <= KR; dk++) {
+                const bool in = ok_j[dj + 1] && ok_i[di + 1] && (DIM == 2 || ok_k[dk + 1]);
+                v[((dj + 1) * 3 + di + 1) * (2 * KR + 1) + dk + KR] = in ? (TA)base[dj * sj + di * si + dk * DIM] : TA(0);
+            }
     TA acc = TA(0);
 #pragma unroll
     for (int dj = -1; dj <= 1; dj++) {
-        const int j = fj + dj;
-        if (j < 0 || j >= gf.nn[1]) continue;
         TA accj = TA(0);
 #pragma unroll
         for (int di = -1; di <= 1; di++) {
-            const int i = fi + di;
-            if (i < 0 || i >= gf.nn[0]) continue;
             TA acci = TA(0);
 #pragma unroll
             for (int dk = -KR; dk <= KR; dk++) {
-                const int k = fk + dk;
-                if (DIM == 3 && (k < 0 || k >= gf.nn[2])) continue;
-                const TA v = (TA)vf[nidx(gf, i, j, k) * DIM + d];
-                acci += dk == 0 ? v : TA(0.5) * v;
+                const TA q = v[((dj + 1) * 3 + di + 1) * (2 * KR + 1) + dk + KR];
+                acci += dk == 0 ? q : TA(0.5) * q;
             }
             accj += di == 0 ? acci : TA(0.5) * acci;
         }
         acc += dj == 0 ? accj : TA(0.5) * accj;
     }
+    if (done) return;
     const TO bc = (TO)(acc * ti * tj * tk);
     vc[c * DIM + d] = bc;
     // first smoothing sweep of the coarse level from x = 0: x = omega * scale / diag * b
-    if (j0.x) j0.x[c * DIM + d] = (TO)((*j0.omega) * j0.scale) * j0.dinv[c * DIM + d] * bc;
+    if (j0.x) j0.x[c * DIM + d] = jw * bc;
 }
 
 // One thread per fine node (all DIM components, contiguous loads of each parent): P =
@@ -177,7 +190,7 @@ __global__ void __launch_bounds__(256) k_prolong_cells(GridDev<3> gf, GridDev<3>
                                                        T* __restrict__ vf, const int* skip) {
     pdl_wait();
     pdl_trigger();
-    if (skip && *skip) return;
+    const int done = skip ? *skip : 0;  // looked at only once the values are on their way
     const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= gc.n_nodes) return;
     int ic, jc, kc;
@@ -214,6 +227,7 @@ __global__ void __launch_bounds__(256) k_prolong_cells(GridDev<3> gf, GridDev<3>
                 z1[a][b][d] = hi[d];
             }
         }
+    if (done) return;
     // y then x stages, written per (di, dj) as the two z-neighbouring fine nodes
 #pragma unroll
     for (int di = 0; di < 2; di++) {
@@ -281,8 +295,8 @@ template int launch_prolong<float>(const Grid&, const float*, float*, const int*
 // block-stencil matvec (levels >= 1): y_n = sum_o A[n,o] u_{n+o}
 // A block covers 32 consecutive nodes; warp w gathers the neighbour offsets 3w..3w+2 for
 // all 32 nodes (coalesced reads of the structure-of-arrays coefficients), the per-warp
-// partial sums meet in shared memory and warp 0 adds them in a fixed order and applies the
-// epilogue.  3D: 9 warps x 3 offsets, 2D: 3 warps x 3 offsets.
+// partial sums meet in shared memory and warp a adds those of component a in a fixed order and
+// applies the epilogue.  3D: 9 warps x 3 offsets, 2D: 3 warps x 3 offsets.
 // HALF: A holds only the centre and the upper offsets o > c (c = NB/2 the centre, stored
 // block q = o - c); a lower offset o < c uses the symmetry of the level operator,
 // A[n, o] = A[n+o, -o]^T, i.e. block q = c - o of the neighbour n+o, transposed.  The
@@ -292,21 +306,35 @@ template int launch_prolong<float>(const Grid&, const float*, float*, const int*
 // each tile's (NB+1)/2 * DIM^2 coefficient rows are one contiguous run (16 KB in 3D FP32),
 // so DRAM streams through it instead of jumping between NH*BS planes of N values.
 // ---------------------------------------------------------------------------------------
-// Launch bounds: FP32 keeps 7 blocks per SM (32 registers); FP64 lets the compiler take 56
-// registers (4 blocks per SM), measured faster than its default 40 for the FP64 solves.
+// Launch bounds: FP32 keeps 7 blocks per SM (32 registers), FP64 4 (56 registers; the 40 that the
+// compiler took by itself measured slower).
+// On the small levels a launch is a chain of latencies: the completion flag, the Jacobi weight
+// and the epilogue's operands (component a by warp a) are loaded before the coefficients, and the
+// flag is looked at when these have arrived.
 template <int DIM, typename T, bool HALF>
-__global__ void __launch_bounds__(DIM == 3 ? 288 : 96, (DIM == 3 && sizeof(T) == 4) ? 7 : 1)
+__global__ void __launch_bounds__(DIM == 3 ? 288 : 96, DIM == 3 ? (sizeof(T) == 4 ? 7 : 4) : 1)
     k_stencil_matvec(GridDev<DIM> g, const T* __restrict__ A, const T* __restrict__ u, Epi<T> epi) {
     pdl_wait();
     pdl_trigger();
     constexpr int NB = DIM == 3 ? 27 : 9, BS = DIM * DIM, NG = NB / 3, C = NB / 2;
     constexpr long long TS = (long long)(C + 1) * BS * 32;  // values per tile of the half copy
     __shared__ T s_part[NG][DIM][32];
-    if (epi.skip && *epi.skip) return;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const long long n = (long long)blockIdx.x * 32 + l;
     const long long N = g.n_nodes;
     const bool valid = n < N;
+    const int done = epi.skip ? *epi.skip : 0;
+    T pb = T(0), px = T(0), pd = T(0), wgt = T(0);
+    const long long gi = n * DIM + w;
+    if (w < DIM && valid) {
+        if (epi.mode != PF_EPI_STORE) pb = epi.b[gi];
+        if (epi.mode == PF_EPI_JACOBI || epi.mode == PF_EPI_JACOBI_ADD) {
+            wgt = epi_omega(epi);
+            pd = epi.dinv[gi];
+            px = epi.x[gi];
+            if (epi.mode == PF_EPI_JACOBI_ADD) px = epi.xadd[gi] + px;
+        }
+    }
     T acc[DIM];
 #pragma unroll
     for (int a = 0; a < DIM; a++) acc[a] = T(0);
@@ -343,32 +371,25 @@ __global__ void __launch_bounds__(DIM == 3 ? 288 : 96, (DIM == 3 && sizeof(T) ==
             }
         }
     }
+    if (done) return;
 #pragma unroll
     for (int a = 0; a < DIM; a++) s_part[w][a][l] = acc[a];
     __syncthreads();
-    if (w != 0) return;
-    double dot = 0.0;
-    if (valid) {
-        const T wgt = epi_omega(epi);
+    if (w >= DIM || !valid) return;
+    T y = s_part[0][w][l];
 #pragma unroll
-        for (int a = 0; a < DIM; a++) {
-            T y = s_part[0][a][l];
-#pragma unroll
-            for (int v = 1; v < NG; v++) y += s_part[v][a][l];
-            const long long gi = n * DIM + a;
-            const T o = epi_apply(epi, gi, y, wgt);
-            epi.out[gi] = o;
-            if (epi.dot_partial) dot += (double)epi.dot_a[gi] * (double)(epi.dot_of_y ? y : o);
-        }
-    }
-    if (epi.dot_partial) {
-        dot = warp_sum(dot);
-        if (l == 0) epi.dot_partial[blockIdx.x] = dot;
-    }
+    for (int v = 1; v < NG; v++) y += s_part[v][w][l];
+    T o = y;
+    if (epi.mode == PF_EPI_RESID)
+        o = pb - y;
+    else if (epi.mode != PF_EPI_STORE)
+        o = px + wgt * pd * (pb - y);
+    epi.out[gi] = o;
 }
 
 template <typename T>
 int launch_stencil_matvec(const Grid& g, const T* A, const T* u, const Epi<T>& epi, cudaStream_t st, bool half) {
+    if (epi.dot_partial) return fail(PF_UNSUPPORTED, "stencil matvec: no fused dot");
     const unsigned nb = (unsigned)((g.n_nodes + 31) / 32);
     pf::count_launch();
     if (g.dim == 3) {
