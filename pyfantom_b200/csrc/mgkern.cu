@@ -178,85 +178,50 @@ __global__ void k_prolong(GridDev<DIM> gf, GridDev<DIM> gc, const T* __restrict_
     for (int d = 0; d < DIM; d++) vf[f * DIM + d] = acc[d] * scale;
 }
 
-// 3D prolongation by cells: one thread per coarse node (ic, jc, kc) writes the up-to-8 fine
-// nodes (2ic + di, 2jc + dj, 2kc + dk), d in {0, 1}, from the up-to-8 coarse nodes
-// (ic + a, jc + b, kc + c).  Each coarse value is read once per thread instead of once per
-// fine child, and each thread writes two contiguous fine nodes (6 values) per (di, dj), so a
-// warp's stores of consecutive kc are contiguous.  Per axis a fine node at 2c takes parent c,
-// one at 2c + 1 the mean of c and c + 1, or c alone past the last coarse node (odd count):
-// the same values as k_prolong.
+// 3D prolongation by rows: the block of coarse row (ic, jc) (or a chunk of it along z) writes the
+// up-to-4 fine rows (2ic + di, 2jc + dj), di, dj in {0, 1}.  Thread s takes component s % 3 of fine
+// node s / 3 along z in each: it forms the z stage in the up-to-4 coarse rows (ic + a, jc + b), then
+// the y and x stages, and its stores are consecutive across the warp.  Per axis a fine node at 2c
+// takes parent c, one at 2c + 1 the mean of c and c + 1, or c alone past the last coarse node
+// (odd count): the same values as k_prolong.
+// Bound by its stores on the fine levels and by latency on the others: one thread per coarse node
+// writing its 2x2x2 children left 24 dependent loads and 24 strided stores to each thread (FP64:
+// 51 -> 35 us onto 256x128x128, 5.6 -> 3.7 us onto 96x48x48, 4.6 -> 1.75 us onto 24x12x12).
 template <typename T>
-__global__ void __launch_bounds__(256) k_prolong_cells(GridDev<3> gf, GridDev<3> gc, const T* __restrict__ vc,
-                                                       T* __restrict__ vf, const int* skip) {
+__global__ void __launch_bounds__(512) k_prolong_rows(GridDev<3> gf, GridDev<3> gc, int chunks, const T* __restrict__ vc,
+                                                      T* __restrict__ vf, const int* skip) {
     pdl_wait();
     pdl_trigger();
     const int done = skip ? *skip : 0;  // looked at only once the values are on their way
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= gc.n_nodes) return;
-    int ic, jc, kc;
-    ndec(gc, c, ic, jc, kc);
+    const unsigned row = blockIdx.x / (unsigned)chunks;
+    const int s = (int)(blockIdx.x - row * (unsigned)chunks) * (int)blockDim.x + (int)threadIdx.x;
+    if (s >= 3 * gf.nn[2]) return;
+    const int jc = (int)(row / (unsigned)gc.nn[0]), ic = (int)(row - (unsigned)jc * (unsigned)gc.nn[0]);
+    const int k = s / 3, d = s - 3 * k, kc = k >> 1;
     auto itw = [](int v, int n) { return (v == 0 || v == n - 1) ? T(1.0 / 1.5) : T(0.5); };
-    const bool hx = ic + 1 < gc.nn[0], hy = jc + 1 < gc.nn[1], hz = kc + 1 < gc.nn[2];  // upper parents
-    const bool fx = 2 * ic + 1 < gf.nn[0], fy = 2 * jc + 1 < gf.nn[1], fz = 2 * kc + 1 < gf.nn[2];  // odd children
-    // z stage for the four (a, b) parent columns: values at fine k = 2kc (z0) and 2kc + 1 (z1)
-    T z0[2][2][3], z1[2][2][3];
+    const bool hx = ic + 1 < gc.nn[0], hy = jc + 1 < gc.nn[1];         // upper parents
+    const bool up = (k & 1) && kc + 1 < gc.nn[2];
+    const T wk0 = itw(kc, gc.nn[2]), wk1 = itw(kc + 1, gc.nn[2]);
+    T z[2][2];  // z stage in row (ic + a, jc + b); a missing row is not used
 #pragma unroll
     for (int a = 0; a < 2; a++)
 #pragma unroll
         for (int b = 0; b < 2; b++) {
-            const bool ok = (a == 0 || hx) && (b == 0 || hy);
-            const int pi = ic + (ok ? a : 0), pj = jc + (ok ? b : 0);
+            const int pi = ic + (hx ? a : 0), pj = jc + (hy ? b : 0);
             const T wab = itw(pi, gc.nn[0]) * itw(pj, gc.nn[1]);
-            const T* v0 = vc + nidx(gc, pi, pj, kc) * 3;
-            const T w0 = wab * itw(kc, gc.nn[2]);
-            T lo[3], hi[3];
-#pragma unroll
-            for (int d = 0; d < 3; d++) lo[d] = ok ? w0 * v0[d] : T(0);
-            if (hz) {
-                const T* v1 = vc + nidx(gc, pi, pj, kc + 1) * 3;
-                const T w1 = wab * itw(kc + 1, gc.nn[2]);
-#pragma unroll
-                for (int d = 0; d < 3; d++) hi[d] = ok ? T(0.5) * (lo[d] + w1 * v1[d]) : T(0);
-            } else {
-#pragma unroll
-                for (int d = 0; d < 3; d++) hi[d] = lo[d];
-            }
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                z0[a][b][d] = lo[d];
-                z1[a][b][d] = hi[d];
-            }
+            const T* v = vc + nidx(gc, pi, pj, kc) * 3 + d;
+            const T lo = wab * wk0 * v[0];
+            z[a][b] = up ? T(0.5) * (lo + wab * wk1 * v[3]) : lo;
         }
     if (done) return;
-    // y then x stages, written per (di, dj) as the two z-neighbouring fine nodes
-#pragma unroll
-    for (int di = 0; di < 2; di++) {
-        if (di && !fx) continue;
-#pragma unroll
-        for (int dj = 0; dj < 2; dj++) {
-            if (dj && !fy) continue;
-            T o0[3], o1[3];
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                // along y for column a, then along x
-                T ya0[2], ya1[2];
-#pragma unroll
-                for (int a = 0; a < 2; a++) {
-                    ya0[a] = dj == 0 ? z0[a][0][d] : (hy ? T(0.5) * (z0[a][0][d] + z0[a][1][d]) : z0[a][0][d]);
-                    ya1[a] = dj == 0 ? z1[a][0][d] : (hy ? T(0.5) * (z1[a][0][d] + z1[a][1][d]) : z1[a][0][d]);
-                }
-                o0[d] = di == 0 ? ya0[0] : (hx ? T(0.5) * (ya0[0] + ya0[1]) : ya0[0]);
-                o1[d] = di == 0 ? ya1[0] : (hx ? T(0.5) * (ya1[0] + ya1[1]) : ya1[0]);
-            }
-            T* out = vf + nidx(gf, 2 * ic + di, 2 * jc + dj, 2 * kc) * 3;
-#pragma unroll
-            for (int d = 0; d < 3; d++) out[d] = o0[d];
-            if (fz) {
-#pragma unroll
-                for (int d = 0; d < 3; d++) out[3 + d] = o1[d];
-            }
-        }
-    }
+    const T y0 = hy ? T(0.5) * (z[0][0] + z[0][1]) : z[0][0], y1 = hy ? T(0.5) * (z[1][0] + z[1][1]) : z[1][0];
+    const bool fx = 2 * ic + 1 < gf.nn[0], fy = 2 * jc + 1 < gf.nn[1];  // odd children
+    T* out = vf + nidx(gf, 2 * ic, 2 * jc, 0) * 3 + s;
+    const long long si = (long long)gf.nn[2] * 3, sj = si * gf.nn[0];
+    out[0] = z[0][0];
+    if (fx) out[si] = hx ? T(0.5) * (z[0][0] + z[1][0]) : z[0][0];
+    if (fy) out[sj] = y0;
+    if (fx && fy) out[sj + si] = hx ? T(0.5) * (y0 + y1) : y0;
 }
 
 template <typename TI, typename TO>
@@ -276,10 +241,11 @@ int launch_prolong(const Grid& gf, const T* vc, T* vf, const int* skip, cudaStre
     const Grid gc = coarse_grid(gf);
     const unsigned nb = (unsigned)((gf.n_nodes + 255) / 256);
     pf::count_launch();
-    if (gf.dim == 3)
-        PF_CUDA(launch_pdl(k_prolong_cells<T>, dim3((unsigned)((gc.n_nodes + 255) / 256)), dim3(256), 0, st,
-                           gdev<3>(gf), gdev<3>(gc), vc, vf, skip));
-    else
+    if (gf.dim == 3) {
+        const int n = 3 * gf.nn[2], chunks = (n + 511) / 512, th = ((n + chunks - 1) / chunks + 31) / 32 * 32;
+        PF_CUDA(launch_pdl(k_prolong_rows<T>, dim3((unsigned)((long long)gc.nn[0] * gc.nn[1] * chunks)), dim3(th), 0, st,
+                           gdev<3>(gf), gdev<3>(gc), chunks, vc, vf, skip));
+    } else
         PF_CUDA(launch_pdl(k_prolong<2, T>, dim3(nb), dim3(256), 0, st, gdev<2>(gf), gdev<2>(gc), vc, vf, skip));
     PF_LAUNCH_CHECK("prolong launch");
     return PF_OK;
