@@ -19,6 +19,8 @@ def to_torch_dtype(dtype) -> torch.dtype:
 
 def as_cuda(x, dtype=None) -> torch.Tensor:
     """Contiguous CUDA tensor view/copy of a tensor, numpy array, DLPack object or scalar list."""
+    if type(x) is torch.Tensor and x.is_cuda and (dtype is None or x.dtype is dtype) and x.is_contiguous():
+        return x
     td = to_torch_dtype(dtype) if dtype is not None else None
     if isinstance(x, torch.Tensor):
         t = x

@@ -147,18 +147,19 @@ class StructuredStiffnessKernel(StiffnessKernel):
         self._refresh_mask()
 
     def _mask_ptr(self):
-        return _lib.ptr(self.node_mask) if self.has_con else _lib.ptr(None)
+        return _lib.ptr(self.node_mask) if self.has_con else None
 
     # --- operator ----------------------------------------------------------------------
     def _matvec(self, rho, vec):
         vec = as_cuda(vec, torch.float64)
-        if self.mat_vec is None or self.mat_vec.shape[0] != self.shape[0]:
-            self.mat_vec = torch.empty(self.shape[0], dtype=torch.float64, device=device())
-        if vec.data_ptr() == self.mat_vec.data_ptr():
+        out = self.mat_vec
+        if out is None or out.shape[0] != self.shape[0]:
+            out = self.mat_vec = torch.empty(self.shape[0], dtype=torch.float64, device=device())
+        if vec.data_ptr() == out.data_ptr():
             vec = vec.clone()
-        _lib.check(_lib.load().pf_matvec_f64(self._op, _lib.ptr(rho), _lib.ptr(vec), self._mask_ptr(),
-                                             _lib.ptr(self.mat_vec), _lib.stream()))
-        return self.mat_vec
+        ptr = _lib.ptr
+        _lib.check(_lib.load().pf_matvec_f64(self._op, ptr(rho), ptr(vec), self._mask_ptr(), ptr(out), _lib.stream()))
+        return out
 
     def _rmatvec(self, rho, vec):
         return self._matvec(rho, vec)
