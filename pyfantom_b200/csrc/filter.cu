@@ -20,6 +20,15 @@
 
 #include "common.cuh"
 
+namespace pf {
+// the tap columns as kernel parameters (uniform loads): cone filters up to rmin 3
+constexpr int kTapCols = 32, kTapWeights = 128;
+struct FilterTaps {
+    int4 col[kTapCols];
+    double w[kTapWeights];
+};
+}  // namespace pf
+
 struct pf_filter {
     pf::Grid grid;
     int n_taps;
@@ -33,6 +42,7 @@ struct pf_filter {
     double* d_cw;      // weights over norm_in, column by column
     int rad[3];        // largest offset along x, y, z (2D: 0, x, y)
     double norm_in;    // normaliser of an element all of whose taps are inside
+    pf::FilterTaps taps;
 };
 
 namespace pf {
@@ -117,13 +127,18 @@ __device__ __forceinline__ void filter_column(const double* s, int plane, const 
 // With 27 taps an output costs 9 (RI + 2) / RI shared-memory reads and 27 FMAs.  Bound by
 // instruction issue (2.4 warp instructions per cycle and SM, 24 % of the FP64 pipe), not by
 // its 16 B of DRAM traffic per element.  256x128x128, rmin 2, forward and adjoint together:
-// 89.7 us against 367 us for k_filter; 96x48x48: 21.5 against 29.7 us (half of it host time).
-// Staging by division-free rows rather than by a flat index took 108 to 97 us, the constant
-// normaliser in the weights 97 to 90 us.
+// 76.4 us against 367 us for k_filter; 96x48x48: 14.2 against 29.7 us.  Staging by division-free
+// rows rather than by a flat index took 108 to 97 us, the constant normaliser in the weights 97 to
+// 90 us, the tap table in the kernel's parameters (uniform loads instead of shared-memory ones)
+// and eight staging loads in flight 90 to 76 us.
 template <int RI, int MI, int TK, bool ADJ>
-__global__ void __launch_bounds__(256) k_filter_tile(const FilterTile t, const int4* __restrict__ col,
-                                                     const double* __restrict__ cw, const double* __restrict__ norm,
-                                                     const double* __restrict__ x, double* __restrict__ y) {
+__global__ void __launch_bounds__(256) k_filter_tile(const FilterTile t, const __grid_constant__ FilterTaps tap,
+                                                     const int4* __restrict__ col, const double* __restrict__ cw,
+                                                     const double* __restrict__ norm, const double* __restrict__ x,
+                                                     double* __restrict__ y) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr bool TAB = MI > 2;  // tap table in shared memory instead of the kernel's parameters
     constexpr int TJ = 256 / TK;
     extern __shared__ __align__(16) double s_f[];
     const int SJ = TJ + 2 * t.rj, SK = TK + 2 * t.rk, plane = SJ * SK, SI = RI + 2 * t.ri;
@@ -132,8 +147,10 @@ __global__ void __launch_bounds__(256) k_filter_tile(const FilterTile t, const i
     const int tid = threadIdx.x, tk = tid % TK, tj = tid / TK;
     const unsigned b = blockIdx.x, bt = b / t.tk;
     const int k0 = (int)(b - bt * t.tk) * TK, j0 = (int)(bt % t.tj) * TJ, i0 = (int)(bt / t.tj) * RI;
-    for (int q = tid; q < t.nw; q += 256) s_w[q] = cw[q];
-    for (int q = tid; q < t.ncol; q += 256) s_c[q] = col[q];
+    if constexpr (TAB) {
+        for (int q = tid; q < t.nw; q += 256) s_w[q] = cw[q];
+        for (int q = tid; q < t.ncol; q += 256) s_c[q] = col[q];
+    }
     // elements with the interior normaliser (already in the weights); `inner`: all staged ones
     auto is_in = [&](int i, int j, int k) {
         return i >= t.ri && i < t.nx - t.ri && j >= t.rj && j < t.ny - t.rj && k >= t.rk && k < t.nz - t.rk;
@@ -155,7 +172,7 @@ __global__ void __launch_bounds__(256) k_filter_tile(const FilterTile t, const i
     const int rows = SI * SJ;
     {
         int a = 0, bj = tj;
-#pragma unroll 4
+#pragma unroll 8
         for (int r = tj; r < rows; r += TJ) {
             stage(a, bj, tk);
             bj += TJ;
@@ -174,15 +191,15 @@ __global__ void __launch_bounds__(256) k_filter_tile(const FilterTile t, const i
     for (int r = 0; r < RI; r++) acc[r] = 0.0;
     const double* base = s_f + (tj + t.rj) * SK + tk + t.rk;
     for (int c = 0; c < t.ncol; c++) {
-        const int4 cc = s_c[c];
+        const int4 cc = TAB ? s_c[c] : tap.col[c];
         const double* sc = base + (t.ri - cc.z) * plane + cc.x * SK + cc.y;
-        const double* wc = s_w + cc.w;
+        const double* wc = TAB ? s_w + cc.w : tap.w + cc.w;
         if (cc.z == 0) filter_column<RI, 0>(sc, plane, wc, acc);
-        if constexpr (MI >= 1)
+        if constexpr (RI > 1 && MI >= 1)
             if (cc.z == 1) filter_column<RI, 1>(sc, plane, wc, acc);
-        if constexpr (MI >= 2)
+        if constexpr (RI > 1 && MI >= 2)
             if (cc.z == 2) filter_column<RI, 2>(sc, plane, wc, acc);
-        if constexpr (MI >= 4) {
+        if constexpr (RI > 1 && MI >= 4) {
             if (cc.z == 3) filter_column<RI, 3>(sc, plane, wc, acc);
             if (cc.z == 4) filter_column<RI, 4>(sc, plane, wc, acc);
         }
@@ -218,8 +235,8 @@ static int launch_filter_tile(const pf_filter* f, FilterTile t, const double* x,
         PF_CUDA(cudaFuncSetAttribute(k_filter_tile<RI, MI, TK, ADJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kFilterMaxSmem));
     count_launch();
-    k_filter_tile<RI, MI, TK, ADJ><<<(unsigned)nb, 256, sm, st>>>(t, reinterpret_cast<const int4*>(f->d_col), f->d_cw,
-                                                                  f->d_norm, x, y);
+    PF_CUDA(launch_pdl(k_filter_tile<RI, MI, TK, ADJ>, dim3((unsigned)nb), dim3(256), sm, st, t, f->taps,
+                       reinterpret_cast<const int4*>(f->d_col), (const double*)f->d_cw, (const double*)f->d_norm, x, y));
     PF_LAUNCH_CHECK("filter launch");
     return PF_OK;
 }
@@ -249,15 +266,17 @@ static int dispatch_filter_tile(const pf_filter* f, const double* x, double* y, 
     const bool long_run = cover(k16 ? 16 : 32) * ((t.nx + 7) / 8) >= 2 * kNumSM;
 #define PF_FT(RI, MI) \
     return k16 ? launch_filter_tile<RI, MI, 16, ADJ>(f, t, x, y, st) : launch_filter_tile<RI, MI, 32, ADJ>(f, t, x, y, st)
-    if (g.dim == 2) PF_FT(1, 0);
-    if (t.ri <= 1) {
+    if (g.dim == 2 && f->ncol <= kTapCols && f->n_taps <= kTapWeights) PF_FT(1, 0);
+    const bool table = f->ncol > kTapCols || f->n_taps > kTapWeights;
+    if (t.ri <= 1 && !table) {
         if (long_run) PF_FT(8, 1);
         PF_FT(4, 1);
     }
-    if (t.ri == 2) {
+    if (t.ri == 2 && !table) {
         if (long_run) PF_FT(8, 2);
         PF_FT(4, 2);
     }
+    if (g.dim == 2) PF_FT(1, 3);
     if (long_run) PF_FT(8, 4);
     PF_FT(4, 4);
 #undef PF_FT
@@ -316,6 +335,10 @@ static void filter_columns(pf_filter* f, const int* off, const double* w, int* h
     f->ncol = t.ncol;
     memcpy(h_col, col.data(), sizeof(int) * col.size());
     memcpy(h_cw, cw.data(), sizeof(double) * cw.size());
+    if (f->ncol <= kTapCols && K <= kTapWeights) {
+        memcpy(f->taps.col, col.data(), sizeof(int) * col.size());
+        memcpy(f->taps.w, cw.data(), sizeof(double) * cw.size());
+    }
 }
 
 static int launch_filter(const pf_filter* f, int mode, const double* x, double* y, cudaStream_t st) {
