@@ -31,17 +31,48 @@ __device__ __forceinline__ void heavy(double r, double beta, double eta, double*
     *dh = beta * (1.0 - t * t) / den;
 }
 
+// r^e: pow, but for the exponents 0 .. 3 of a penalty of 1 to 4 and its derivative, products (at
+// most two roundings, within pow's own error; pow costs some hundred instructions)
+template <int EXP>
+__device__ __forceinline__ double simp_pow(double r, double e) {
+    if (EXP == 0) return 1.0;
+    if (EXP == 1) return r;
+    if (EXP == 2) return r * r;
+    if (EXP == 3) return r * r * r;
+    return pow(r, e);
+}
+
+// PEN: the penalty if it is 1, 2 or 3, else 0.  Bound by FP64 arithmetic: 128x64x64 elements with
+// projection 6.5 us against 12.3 us with pow and three tanh for each element.  The two constant
+// tanh are formed here, once per block, and not on the host: at rho = 0 the projection is
+// tanh(beta eta) + tanh(-beta eta), which cancels to 0 only if both come from one function.
+template <int PEN>
 __global__ void k_penalize(long long n, const double* __restrict__ rho, pf_simp_params P, double* __restrict__ E,
                            double* __restrict__ dE) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ double s_th, s_den;
+    if (P.heavyside) {
+        if (threadIdx.x == 0) {
+            s_th = tanh(P.beta * P.eta);
+            s_den = s_th + tanh(P.beta * (1.0 - P.eta));
+        }
+        __syncthreads();
+    }
+    const double th = P.heavyside ? s_th : 0.0, den = P.heavyside ? s_den : 1.0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         double r = rho[i], dh = 1.0;
-        if (P.heavyside) heavy(rho[i], P.beta, P.eta, &r, &dh);
+        if (P.heavyside) {
+            const double t = tanh(P.beta * (r - P.eta));
+            r = (th + t) / den;
+            dh = P.beta * (1.0 - t * t) / den;
+        }
         if (E) {
-            double e = pow(r, P.penalty);
+            double e = simp_pow<PEN ? PEN : 9>(r, P.penalty);
             e = fmin(fmax(e, P.void_value), 1.0) * P.E_mul;
             E[i] = fmax(e, P.void_value);
         }
-        if (dE) dE[i] = P.penalty * pow(r, P.penalty - 1.0) * dh * P.E_mul;
+        if (dE) dE[i] = P.penalty * simp_pow<PEN ? PEN - 1 : 9>(r, P.penalty - 1.0) * dh * P.E_mul;
     }
 }
 
@@ -776,7 +807,9 @@ extern "C" int pf_penalize_f64(long long n, const double* rho, const pf_simp_par
     if (n < 0 || !rho || !p || (!E && !dE)) return fail(PF_BAD_ARG, "pf_penalize_f64: bad argument");
     if (n == 0) return PF_OK;
     pf::count_launch();
-    k_penalize<<<grid_for(n), kRT, 0, as_stream(stream)>>>(n, rho, *p, E, dE);
+    const double e = p->penalty;
+    auto kernel = e == 1.0 ? k_penalize<1> : e == 2.0 ? k_penalize<2> : e == 3.0 ? k_penalize<3> : k_penalize<0>;
+    PF_CUDA(launch_pdl(kernel, dim3(grid_for(n)), dim3(kRT), 0, as_stream(stream), n, rho, *p, E, dE));
     PF_LAUNCH_CHECK("penalize launch");
     return PF_OK;
 }

@@ -193,3 +193,35 @@ def test_direct_band(lib, nel):
                                  lib.stream()) == lib.PF_FACTOR_FAILED
     L.pf_direct_destroy(d)
     L.pf_op_destroy(op)
+
+
+@pytest.mark.parametrize("nel", [(1, 1, 1), (2, 3, 31), (17, 2, 32), (33, 5, 33), (16, 9, 64), (50, 20, 70)])
+def test_sensitivity_march(lib, nel):
+    # z remainders of the 32-wide march and chunk ends along x; 24-term quadratic forms: 1e-13
+    from conftest import unit_K0
+    K0 = np.ascontiguousarray(unit_K0(3, h=(1.0, 1.25, 0.8)))
+    U = np.random.default_rng(5).standard_normal(O.n_nodes(nel) * 3)
+    L = lib.load()
+    grid, op = lib.make_grid(nel), ctypes.c_void_p()
+    lib.check(L.pf_op_create(ctypes.byref(grid), K0.ctypes.data, ctypes.byref(op)))
+    Ut = T(U)
+    dk = torch.full((O.n_elem(nel),), np.nan, dtype=torch.float64, device="cuda")
+    lib.check(L.pf_sensitivity_f64(op, lib.ptr(Ut), lib.ptr(dk), lib.stream()))
+    assert rel(N(dk), O.process_dk(nel, K0, U)) < 1e-13
+    L.pf_op_destroy(op)
+
+
+@pytest.mark.parametrize("p", [1.0, 2.0, 3.0])
+@pytest.mark.parametrize("heavyside", [False, True])
+def test_penalize_whole_exponents_equal_pow(lib, p, heavyside):
+    # the products against the general route, one ulp of the penalty away: r^(p eps) moves by at
+    # most 3 * ln(1e9) * 2.2e-16 = 1.4e-14, pow and the products by a few ulp more
+    from pyfantom_b200.Problem import penalize_device, simp_params
+    rho = T(np.concatenate([[0.0, 1.0], np.random.default_rng(2).uniform(1e-9, 1, 5000)]))
+    E, dE = penalize_device(rho, simp_params(p, 1e-9, 1.5, 3.0, 0.45, heavyside), True, True)
+    E2, dE2 = penalize_device(rho, simp_params(np.nextafter(p, 9.0), 1e-9, 1.5, 3.0, 0.45, heavyside), True, True)
+    assert np.allclose(N(E), N(E2), rtol=2e-14, atol=0)
+    # (at rho = 0 with p = 1 the derivative is r^0 = 1 here and r^(2e-16) = 0 there)
+    assert np.allclose(N(dE)[1:], N(dE2)[1:], rtol=2e-14, atol=0)
+    # an empty projected density is exactly void in either route
+    assert float(E[0]) == float(E2[0]) == 1e-9 * 1.5
