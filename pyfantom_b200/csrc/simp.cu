@@ -560,9 +560,11 @@ __global__ void __launch_bounds__(kRT, 2) k_oc_pass(long long n, const double* _
         // the sums of the elements decided for the bracket of the building pass, then the others
         double* head = reinterpret_cast<double*>(seg);
         const int cnt = seg[4];
+        int next = 6 + l < lcap ? seg[6 + l] : 0;  // the first entry beside the count
         if (l == 0) cst = head[0], lin = head[1];
         for (int q = l; q < cnt; q += 32) {
-            const int i = seg[6 + q];
+            const int i = next;
+            if (q + 32 < cnt) next = seg[6 + q + 32];
             oc_accumulate<kOcMid>(x[i], allzero ? 1e-3 : ocp[i], dg[i], move, s_r, rlo, rhi, cst, lin, acc);
         }
     } else if (mode == 2) {
@@ -602,12 +604,14 @@ __global__ void __launch_bounds__(kRT, 2) k_oc_pass(long long n, const double* _
     if (!s_last) return;
     __threadfence();
     {  // thread (t, group): every 16th block's sum for midpoint t
-        const int t = tid & 15;
-        double s = 0.0;
-        if (t < ne) {
-#pragma unroll 4
-            for (unsigned b = tid >> 4; b < gridDim.x; b += kRT / 16) s += __ldcg(partials + (long long)b * kOcMid + t);
-        }
+        constexpr int G = kRT / 16, NL = (2 * kNumSM + G - 1) / G;  // at most 2 blocks per SM (oc_blocks)
+        const int t = tid & 15, tc = t < ne ? t : 0, nbk = (int)gridDim.x;
+        double part[NL], s = 0.0;  // all loads in flight together
+#pragma unroll
+        for (int q = 0; q < NL; q++) part[q] = __ldcg(partials + (long long)min((tid >> 4) + q * G, nbk - 1) * kOcMid + tc);
+#pragma unroll
+        for (int q = 0; q < NL; q++)
+            if ((tid >> 4) + q * G < nbk) s += part[q];
         s += __shfl_xor_sync(0xffffffffu, s, 16);
         if (l < 16) s_part[w][t] = s;  // 17 columns a row
     }
