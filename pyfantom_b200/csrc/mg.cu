@@ -31,6 +31,7 @@ namespace pf {
 
 constexpr int kMaxLevel = 12;
 constexpr int kRedThreads = 256;
+constexpr int kWide = 6;  // blocks per SM of the vector kernels with up to 42 registers
 
 struct PcgState {
     double rho_old, norm_b, alpha, beta, R, omega;
@@ -286,7 +287,7 @@ struct CompIter {
 // x += alpha p, then p = z + beta p (init: p = z alone); with the deflation field yf, z - Q coef
 // in place of z.  After the iteration that ends the solve only x is still to be updated (xlag).
 template <typename TZ>
-__global__ void __launch_bounds__(kRedThreads) k_pcg_p(long long n, const TZ* __restrict__ z, double* __restrict__ p,
+__global__ void __launch_bounds__(kRedThreads, kWide) k_pcg_p(long long n, const TZ* __restrict__ z, double* __restrict__ p,
                                                        double* __restrict__ x, const PcgState* st, int init,
                                                        const float* __restrict__ yf, int dof) {
     pdl_wait();
@@ -463,7 +464,7 @@ __global__ void k_defl_xadd(long long n, int dof, const float* __restrict__ yf, 
 }
 // partials of r.z (index 0) and t_d = W_d . z (indices 1..3)
 template <typename TZ>
-__global__ void __launch_bounds__(kRedThreads) k_dot_defl(long long n, const double* __restrict__ r,
+__global__ void __launch_bounds__(kRedThreads, kWide) k_dot_defl(long long n, const double* __restrict__ r,
                                                           const TZ* __restrict__ z, const double* __restrict__ Wd,
                                                           double* partials, const int* skip) {
     pdl_wait();
@@ -486,9 +487,12 @@ __global__ void __launch_bounds__(kRedThreads) k_dot_defl(long long n, const dou
     }
 }
 
-static unsigned vec_blocks(long long n) {
+// Grid of a vector kernel: one wave of per_sm blocks on every SM, which its registers must allow
+// (8 of 256 threads up to 32 registers, 6 up to 42): a second, partly empty wave of 1184 blocks
+// where 888 fit cost k_dot_defl and k_pcg_p up to a quarter of their time.
+static unsigned vec_blocks(long long n, int per_sm = 8) {
     long long nb = (n + kRedThreads - 1) / kRedThreads;
-    const long long cap = 8LL * kNumSM;
+    const long long cap = (long long)per_sm * kNumSM;
     if (nb > cap) nb = cap;
     if (nb < 1) nb = 1;
     return (unsigned)nb;
@@ -938,7 +942,8 @@ extern "C" int pf_mg_vcycle(pf_mg* mg, const double* r, double* z, double omega,
 static int precondition(pf_mg* mg, const void** z_out, int step, cudaStream_t st, bool r32_ready) {
     const long long n = mg->L[0].ndof;
     const int* skip = &mg->st->done;
-    long long np = vec_blocks(n);
+    const dim3 wide(vec_blocks(n, kWide));
+    long long np = mg->defl ? vec_blocks(n, kWide) : vec_blocks(n);
     const dim3 vb(vec_blocks(n)), th(kRedThreads);
     int s;
     if (mg->fp32) {
@@ -950,7 +955,7 @@ static int precondition(pf_mg* mg, const void** z_out, int step, cudaStream_t st
         if ((s = vcycle<float>(mg, 0, (const float*)mg->L[0].b, &res, nullptr, nullptr, st))) return s;
         pf::count_launch();
         if (mg->defl)  // r.z and W^T z
-            PF_CUDA(launch_pdl(k_dot_defl<float>, vb, th, 0, st, n, (const double*)mg->r, (const float*)res,
+            PF_CUDA(launch_pdl(k_dot_defl<float>, wide, th, 0, st, n, (const double*)mg->r, (const float*)res,
                                (const double*)mg->Wd, mg->partials, skip));
         else
             PF_CUDA(launch_pdl(k_dot_partial<float>, vb, th, 0, st, n, mg->r, res, mg->partials, skip));
@@ -961,7 +966,7 @@ static int precondition(pf_mg* mg, const void** z_out, int step, cudaStream_t st
         if (mg->defl) {
             if ((s = vcycle<double>(mg, 0, mg->r, &res, nullptr, nullptr, st))) return s;
             pf::count_launch();
-            PF_CUDA(launch_pdl(k_dot_defl<double>, vb, th, 0, st, n, (const double*)mg->r, (const double*)res,
+            PF_CUDA(launch_pdl(k_dot_defl<double>, wide, th, 0, st, n, (const double*)mg->r, (const double*)res,
                                (const double*)mg->Wd, mg->partials, skip));
             PF_LAUNCH_CHECK("dot launch");
         } else if ((s = vcycle<double>(mg, 0, mg->r, &res, mg->partials, mg->r, st))) {
@@ -979,7 +984,7 @@ static int precondition(pf_mg* mg, const void** z_out, int step, cudaStream_t st
 
 static int update_p(pf_mg* mg, const void* z, double* x, int init, cudaStream_t st) {
     const long long n = mg->L[0].ndof;
-    const dim3 vb(vec_blocks(n)), th(kRedThreads);
+    const dim3 vb(vec_blocks(n, kWide)), th(kRedThreads);
     const float* yf = mg->defl ? mg->yf : nullptr;
     pf::count_launch();
     if (mg->fp32)
@@ -1219,7 +1224,7 @@ extern "C" int pf_cg_solve(const pf_op* op, const double* E, const uint8_t* node
     PF_CUDA(launch_pdl(k_dot_partial<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, r, partials, skip));
     PF_CUDA(take(PCG_RHO0, vb));
     pf::count_launch();
-    PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, p, x, S, 1, (const float*)nullptr, 3));
+    PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vec_blocks(n, kWide)), dim3(kRedThreads), 0, st, n, r, p, x, S, 1, (const float*)nullptr, 3));
     PF_LAUNCH_CHECK("cg start");
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -1241,7 +1246,7 @@ extern "C" int pf_cg_solve(const pf_op* op, const double* E, const uint8_t* node
             PF_CUDA(launch_pdl(k_pcg_r, dim3(vb), dim3(kRedThreads), 0, st, n, q, r, S, partials, (float*)nullptr));
             PF_CUDA(take(PCG_CHECK_BETA, vb));
             pf::count_launch();
-            PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vb), dim3(kRedThreads), 0, st, n, r, p, x, S, 0, (const float*)nullptr, 3));
+            PF_CUDA(launch_pdl(k_pcg_p<double>, dim3(vec_blocks(n, kWide)), dim3(kRedThreads), 0, st, n, r, p, x, S, 0, (const float*)nullptr, 3));
         }
         PF_LAUNCH_CHECK("cg iteration");
         it += chunk;

@@ -186,8 +186,10 @@ __global__ void k_prolong(GridDev<DIM> gf, GridDev<DIM> gc, const T* __restrict_
 // (odd count): the same values as k_prolong.
 // Bound by its stores on the fine levels and by latency on the others: one thread per coarse node
 // writing its 2x2x2 children left 24 dependent loads and 24 strided stores to each thread (FP64:
-// 51 -> 35 us onto 256x128x128, 5.6 -> 3.7 us onto 96x48x48, 4.6 -> 1.75 us onto 24x12x12).
-template <typename T>
+// 51 -> 28 us onto 256x128x128, 5.6 -> 3.4 us onto 96x48x48, 4.6 -> 1.75 us onto 24x12x12).
+// NI coarse rows along x per thread (4 on the fine levels: consecutive rows share their parents, and
+// 16 stores are in flight; one row per thread took 33.6 us onto 256x128x128 in FP32).
+template <typename T, int NI>
 __global__ void __launch_bounds__(512) k_prolong_rows(GridDev<3> gf, GridDev<3> gc, int chunks, const T* __restrict__ vc,
                                                       T* __restrict__ vf, const int* skip) {
     pdl_wait();
@@ -196,32 +198,40 @@ __global__ void __launch_bounds__(512) k_prolong_rows(GridDev<3> gf, GridDev<3> 
     const unsigned row = blockIdx.x / (unsigned)chunks;
     const int s = (int)(blockIdx.x - row * (unsigned)chunks) * (int)blockDim.x + (int)threadIdx.x;
     if (s >= 3 * gf.nn[2]) return;
-    const int jc = (int)(row / (unsigned)gc.nn[0]), ic = (int)(row - (unsigned)jc * (unsigned)gc.nn[0]);
+    const int nxb = (gc.nn[0] + NI - 1) / NI;
+    const int jc = (int)(row / (unsigned)nxb), ic0 = (int)(row - (unsigned)jc * (unsigned)nxb) * NI;
     const int k = s / 3, d = s - 3 * k, kc = k >> 1;
     auto itw = [](int v, int n) { return (v == 0 || v == n - 1) ? T(1.0 / 1.5) : T(0.5); };
-    const bool hx = ic + 1 < gc.nn[0], hy = jc + 1 < gc.nn[1];         // upper parents
+    const bool hy = jc + 1 < gc.nn[1];  // upper parent along y
     const bool up = (k & 1) && kc + 1 < gc.nn[2];
     const T wk0 = itw(kc, gc.nn[2]), wk1 = itw(kc + 1, gc.nn[2]);
-    T z[2][2];  // z stage in row (ic + a, jc + b); a missing row is not used
+    T z[NI + 1][2];  // z stage in row (ic0 + a, jc + b); a row outside is not used
 #pragma unroll
-    for (int a = 0; a < 2; a++)
+    for (int a = 0; a <= NI; a++)
 #pragma unroll
         for (int b = 0; b < 2; b++) {
-            const int pi = ic + (hx ? a : 0), pj = jc + (hy ? b : 0);
+            const int pi = min(ic0 + a, gc.nn[0] - 1), pj = jc + (hy ? b : 0);
             const T wab = itw(pi, gc.nn[0]) * itw(pj, gc.nn[1]);
             const T* v = vc + nidx(gc, pi, pj, kc) * 3 + d;
             const T lo = wab * wk0 * v[0];
             z[a][b] = up ? T(0.5) * (lo + wab * wk1 * v[3]) : lo;
         }
     if (done) return;
-    const T y0 = hy ? T(0.5) * (z[0][0] + z[0][1]) : z[0][0], y1 = hy ? T(0.5) * (z[1][0] + z[1][1]) : z[1][0];
-    const bool fx = 2 * ic + 1 < gf.nn[0], fy = 2 * jc + 1 < gf.nn[1];  // odd children
-    T* out = vf + nidx(gf, 2 * ic, 2 * jc, 0) * 3 + s;
+    const bool fy = 2 * jc + 1 < gf.nn[1];  // odd child along y
+    T* out = vf + nidx(gf, 2 * ic0, 2 * jc, 0) * 3 + s;
     const long long si = (long long)gf.nn[2] * 3, sj = si * gf.nn[0];
-    out[0] = z[0][0];
-    if (fx) out[si] = hx ? T(0.5) * (z[0][0] + z[1][0]) : z[0][0];
-    if (fy) out[sj] = y0;
-    if (fx && fy) out[sj + si] = hx ? T(0.5) * (y0 + y1) : y0;
+#pragma unroll
+    for (int a = 0; a < NI; a++, out += 2 * si) {
+        const int ic = ic0 + a;
+        if (ic >= gc.nn[0]) break;
+        const bool hx = ic + 1 < gc.nn[0], fx = 2 * ic + 1 < gf.nn[0];
+        const T y0 = hy ? T(0.5) * (z[a][0] + z[a][1]) : z[a][0];
+        const T y1 = hy ? T(0.5) * (z[a + 1][0] + z[a + 1][1]) : z[a + 1][0];
+        out[0] = z[a][0];
+        if (fx) out[si] = hx ? T(0.5) * (z[a][0] + z[a + 1][0]) : z[a][0];
+        if (fy) out[sj] = y0;
+        if (fx && fy) out[sj + si] = hx ? T(0.5) * (y0 + y1) : y0;
+    }
 }
 
 template <typename TI, typename TO>
@@ -243,8 +253,11 @@ int launch_prolong(const Grid& gf, const T* vc, T* vf, const int* skip, cudaStre
     pf::count_launch();
     if (gf.dim == 3) {
         const int n = 3 * gf.nn[2], chunks = (n + 511) / 512, th = ((n + chunks - 1) / chunks + 31) / 32 * 32;
-        PF_CUDA(launch_pdl(k_prolong_rows<T>, dim3((unsigned)((long long)gc.nn[0] * gc.nn[1] * chunks)), dim3(th), 0, st,
-                           gdev<3>(gf), gdev<3>(gc), chunks, vc, vf, skip));
+        // four rows per thread once that still gives every SM eight blocks
+        const bool four = (long long)((gc.nn[0] + 3) / 4) * gc.nn[1] * chunks >= 8LL * kNumSM;
+        const long long rows = (long long)(four ? (gc.nn[0] + 3) / 4 : gc.nn[0]) * gc.nn[1];
+        PF_CUDA(launch_pdl(four ? k_prolong_rows<T, 4> : k_prolong_rows<T, 1>, dim3((unsigned)(rows * chunks)), dim3(th), 0,
+                           st, gdev<3>(gf), gdev<3>(gc), chunks, vc, vf, skip));
     } else
         PF_CUDA(launch_pdl(k_prolong<2, T>, dim3(nb), dim3(256), 0, st, gdev<2>(gf), gdev<2>(gc), vc, vf, skip));
     PF_LAUNCH_CHECK("prolong launch");
