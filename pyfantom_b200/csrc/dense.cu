@@ -5,7 +5,8 @@
 // coarse right-hand side to the host and back.  Here the factorisation stays on the GPU:
 // a right-looking blocked Cholesky with 32x32 tiles (diagonal tile in shared memory,
 // triangular solve of the panel, symmetric rank-32 update of the trailing matrix),
-// followed by the inverse of the factor and the explicit inverse A^-1 = L^-T L^-1.  A
+// followed by the inverse of the factor and the explicit inverse A^-1 = L^-T L^-1; orders up to
+// kGjTiles tiles are inverted directly by a block Gauss-Jordan elimination (k_gj_step).  A
 // coarse solve is then one dense matrix-vector product, spread over many warps, with no
 // host round trip.
 #include "common.cuh"
@@ -144,6 +145,117 @@ __global__ void __launch_bounds__(1024) k_ainv(const double* Linv, double* Ainv,
     Ainv[(long long)(a * TB + ty) * np + b * TB + tx] = s;
 }
 
+// One step p of the block Gauss-Jordan inversion, src -> dst (every tile): with P = src_pp^-1 and
+// W_j = P src_pj (j != p) or P (j = p), tile (i, j) becomes W_j for i = p and
+// (j == p ? 0 : src_ij) - src_ip W_j else.  Each block forms P again (the inverse of a 32 x 32
+// tile, a chain of 32 pivots), so a step is one launch; positive pivots are those of Cholesky.
+// A chain of latencies, about 6 us a step: the inverse of order 675 takes 0.15 ms, where the
+// Cholesky factor, its inverse and their product took 1.6 ms in 88 dependent launches.
+constexpr int kGjTiles = 64;
+constexpr int GP = 36;  // row pitch of the staged tiles (conflict-free MMA fragments)
+__global__ void __launch_bounds__(256) k_gj_step(const double* __restrict__ src, double* __restrict__ dst, int np, int p,
+                                                 double beta, int n, int* fail) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ __align__(16) double sP[TB * GP], sX[TB * GP], sA[TB * GP], s_row[2][TB];
+    const int i = blockIdx.y, j = blockIdx.x, tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+    const int r = tid >> 3, c4 = (tid & 7) * 4;  // this thread's row and four columns
+    auto load = [&](int a, int b) {
+        const double2* t = reinterpret_cast<const double2*>(src + (long long)(a * TB + r) * np + b * TB + c4);
+        const double2 x = t[0], y = t[1];
+        double4 v = {x.x, x.y, y.x, y.y};
+        if (p == 0 && a == b && r >= c4 && r < c4 + 4) {  // the shift, and ones on the padding
+            const double d = a * TB + r < n ? beta : 1.0;
+            if (r == c4) v.x += d;
+            if (r == c4 + 1) v.y += d;
+            if (r == c4 + 2) v.z += d;
+            if (r == c4 + 3) v.w += d;
+        }
+        return v;
+    };
+    auto stage = [&](double* s, double4 v) {
+        *reinterpret_cast<double2*>(s + r * GP + c4) = make_double2(v.x, v.y);
+        *reinterpret_cast<double2*>(s + r * GP + c4 + 2) = make_double2(v.z, v.w);
+    };
+    const double4 d4 = load(p, p);
+    double v[4] = {d4.x, d4.y, d4.z, d4.w};
+    if (j != p) stage(sX, load(p, j));
+    if (i != p) stage(sA, load(i, p));
+    const double4 c0 = (i != p && j != p) ? load(i, j) : double4{0.0, 0.0, 0.0, 0.0};
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < TB; k++) {
+        double* row = s_row[k & 1];
+        if (r == k) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) row[c4 + q] = v[q];
+        }
+        __syncthreads();
+        double piv = row[k];
+        if (!(piv > 0.0)) {
+            if (!bad && tid == 0 && i == p && j == p) atomicCAS(fail, 0, p * TB + k + 1);
+            bad = true;
+            piv = 1.0;
+        }
+        const double inv = 1.0 / piv;
+        const double f = __shfl_sync(0xffffffffu, v[k & 3], (l & 24) | (k >> 2)) * inv;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const double rv = row[c4 + q];
+            const bool diag = c4 + q == k;
+            if (r == k)
+                v[q] = diag ? inv : rv * inv;
+            else
+                v[q] = diag ? -f : fma(-f, rv, v[q]);
+        }
+    }
+    stage(sP, double4{v[0], v[1], v[2], v[3]});
+    __syncthreads();
+    // 32 x 32 products by 8 x 8 x 4 FP64 MMAs: warp w takes rows 8 (w >> 1), columns 16 (w & 1) on
+    const int fr = l >> 2, fk = l & 3, r0 = 8 * (w >> 1), n0 = 16 * (w & 1);
+    auto mma = [&](double (&acc)[2][2], const double* A, const double* B, double sign) {
+#pragma unroll
+        for (int kk = 0; kk < TB; kk += 4) {
+            const double a = sign * A[(r0 + fr) * GP + kk + fk];
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
+                const double b = B[(kk + fk) * GP + n0 + 8 * t + fr];
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                    : "+d"(acc[t][0]), "+d"(acc[t][1])
+                    : "d"(a), "d"(b));
+            }
+        }
+    };
+    const double* W = sP;
+    if (j != p) {
+        double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        mma(acc, sP, sX, 1.0);
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < 2; t++)
+            *reinterpret_cast<double2*>(sX + (r0 + fr) * GP + n0 + 8 * t + 2 * fk) = make_double2(acc[t][0], acc[t][1]);
+        W = sX;
+        __syncthreads();
+    }
+    double* out = dst + (long long)(i * TB) * np + j * TB;
+    if (i == p) {
+        const double2 x = *reinterpret_cast<const double2*>(W + r * GP + c4), y = *reinterpret_cast<const double2*>(W + r * GP + c4 + 2);
+        *reinterpret_cast<double2*>(out + (long long)r * np + c4) = x;
+        *reinterpret_cast<double2*>(out + (long long)r * np + c4 + 2) = y;
+        return;
+    }
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    mma(acc, sA, W, -1.0);
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+        *reinterpret_cast<double2*>(sP + (r0 + fr) * GP + n0 + 8 * t + 2 * fk) = make_double2(acc[t][0], acc[t][1]);
+    __syncthreads();
+    const double2 x = *reinterpret_cast<const double2*>(sP + r * GP + c4), y = *reinterpret_cast<const double2*>(sP + r * GP + c4 + 2);
+    *reinterpret_cast<double2*>(out + (long long)r * np + c4) = make_double2(c0.x + x.x, c0.y + x.y);
+    *reinterpret_cast<double2*>(out + (long long)r * np + c4 + 2) = make_double2(c0.z + y.x, c0.w + y.y);
+}
+
 // x = Ainv b (rows < n), one warp per row, accumulation in FP64
 template <typename T>
 __global__ void __launch_bounds__(256) k_dense_matvec(const double* __restrict__ Ainv, int np, int n,
@@ -211,6 +323,20 @@ int dense_factor_linv(Dense* d, double beta, cudaStream_t st) {
 }
 
 int dense_factor_invert(Dense* d, double beta, cudaStream_t st) {
+    if (d->np <= kGjTiles * TB) {
+        // M -> Linv -> M ..., the last step into Ainv
+        const int nt = d->np / TB;
+        PF_CUDA(cudaMemsetAsync(d->fail, 0, sizeof(int), st));
+        const double* src = d->M;
+        for (int p = 0; p < nt; p++) {
+            double* dst = p + 1 == nt ? d->Ainv : src == d->M ? d->Linv : d->M;
+            pf::count_launch();
+            PF_CUDA(launch_pdl(k_gj_step, dim3(nt, nt), dim3(256), 0, st, src, dst, d->np, p, beta, d->n, d->fail));
+            src = dst;
+        }
+        PF_LAUNCH_CHECK("coarse inversion launch");
+        return PF_OK;
+    }
     int s = dense_factor_linv(d, beta, st);
     if (s) return s;
     const int np = d->np, nt = np / TB;

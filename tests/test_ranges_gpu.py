@@ -225,3 +225,29 @@ def test_penalize_whole_exponents_equal_pow(lib, p, heavyside):
     assert np.allclose(N(dE)[1:], N(dE2)[1:], rtol=2e-14, atol=0)
     # an empty projected density is exactly void in either route
     assert float(E[0]) == float(E2[0]) == 1e-9 * 1.5
+
+
+@pytest.mark.parametrize("nel,n_level", [((8, 4, 4), 2), ((24, 12, 12), 2), ((16, 14, 14), 1), ((20, 20, 20), 1), ((40, 24), 2),
+                                         ((120, 90), 1)])
+def test_coarse_inverse(lib, nel, n_level):
+    # one V-cycle against the oracle's (dense Cholesky of the coarsest operator), whose coarsest
+    # orders run from two tiles through both routes (an order of 6,144 is the limit);
+    # the two solves differ by the coarse operator's condition (up to 1e5) times 1e-16: 1e-9
+    from conftest import unit_K0
+    from pyfantom_b200 import workloads
+    from pyfantom_b200.CUDA import MultiGrid, StructuredMesh2D, StructuredMesh3D, StructuredStiffnessKernel
+    from pyfantom_b200.physics import LinearElasticity
+    dim = len(nel)
+    mesh = (StructuredMesh3D if dim == 3 else StructuredMesh2D)(*nel, *nel, physics=LinearElasticity(E=1.0, nu=0.3))
+    kern = StructuredStiffnessKernel(mesh)
+    wl = workloads.cantilever3d(*nel) if dim == 3 else workloads.mbb2d(*nel)
+    kern.add_constraints(T(wl["fixed_dofs"], torch.int64))
+    rng = np.random.default_rng(1)
+    E = rng.uniform(0.1, 1.0, O.n_elem(nel))
+    kern.set_rho(T(E))
+    s = MultiGrid(mesh, kern, n_smooth=2, omega=0.6, n_level=n_level, coarse_op="stencil")
+    s.setup()
+    r = rng.standard_normal(kern.shape[0])
+    r[wl["fixed_dofs"]] = 0.0
+    z = N(s.vcycle(T(r), omega=0.4))
+    assert rel(z, O.mg_vcycle(nel, unit_K0(dim), E, wl["fixed_dofs"], r, n_level=n_level, omega=0.4)) < 1e-9
