@@ -75,67 +75,129 @@ static GridDev<DIM> gdev(const Grid& g) {
 // ---------------------------------------------------------------------------------------
 // transfers
 // ---------------------------------------------------------------------------------------
-// One thread per (coarse node, component): the 3^DIM weighted fine values of that
+// 2D restriction, one thread per (coarse node, component): the 9 weighted fine values of that
 // component, accumulated in the output precision.  Per axis the weights are 0.5 / 1 / 0.5
 // and 1/tw factorises into 1/1.5 (boundary node) or 1/2.
-template <int DIM, typename TI, typename TO>
-__global__ void k_restrict(GridDev<DIM> gf, GridDev<DIM> gc, const TI* __restrict__ vf, TO* __restrict__ vc,
-                           const int* skip, Jacobi0<TO> j0) {
+template <typename TI, typename TO>
+__global__ void k_restrict_q(GridDev<2> gf, GridDev<2> gc, const TI* __restrict__ vf, TO* __restrict__ vc,
+                             const int* skip, Jacobi0<TO> j0) {
     pdl_wait();
     pdl_trigger();
-    using TA = TO;  // accumulation precision
     const int done = skip ? *skip : 0;  // looked at only once the values are on their way
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= gc.n_nodes * DIM) return;
-    const long long c = (unsigned)t / DIM;
-    const int d = (int)(t - c * DIM);
+    if (t >= gc.n_nodes * 2) return;
+    const long long c = (unsigned)t / 2;
+    const int d = (int)(t - c * 2);
     TO jw = TO(0);
-    if (j0.x) jw = (TO)((*j0.omega) * j0.scale) * j0.dinv[c * DIM + d];
+    if (j0.x) jw = (TO)((*j0.omega) * j0.scale) * j0.dinv[t];
     int ic, jc, kc;
     ndec(gc, c, ic, jc, kc);
-    const int fi = 2 * ic, fj = 2 * jc, fk = 2 * kc;
-    const TA ti = (ic == 0 || ic == gc.nn[0] - 1) ? TA(1.0 / 1.5) : TA(0.5);
-    const TA tj = (jc == 0 || jc == gc.nn[1] - 1) ? TA(1.0 / 1.5) : TA(0.5);
-    TA tk = TA(1);
-    if (DIM == 3) tk = (kc == 0 || kc == gc.nn[2] - 1) ? TA(1.0 / 1.5) : TA(0.5);
-    constexpr int KR = DIM == 3 ? 1 : 0;
+    const int fi = 2 * ic, fj = 2 * jc;
+    const TO ti = (ic == 0 || ic == gc.nn[0] - 1) ? TO(1.0 / 1.5) : TO(0.5);
+    const TO tj = (jc == 0 || jc == gc.nn[1] - 1) ? TO(1.0 / 1.5) : TO(0.5);
     // values outside the grid are not read but their place in the sums is kept, so that the loads
     // need no branches and are all in flight together
-    TA v[DIM == 3 ? 27 : 9];
+    TO v[9];
     const bool ok_i[3] = {fi > 0, true, fi + 1 < gf.nn[0]}, ok_j[3] = {fj > 0, true, fj + 1 < gf.nn[1]};
-    const bool ok_k[3] = {fk > 0, true, fk + 1 < gf.nn[2]};
-    const TI* base = vf + nidx(gf, fi, fj, fk) * DIM + d;
-    const int si = DIM == 3 ? gf.nn[2] * DIM : DIM, sj = si * gf.nn[0];
+    const TI* base = vf + nidx(gf, fi, fj, 0) * 2 + d;
+    const int sj = 2 * gf.nn[0];
 #pragma unroll
     for (int dj = -1; dj <= 1; dj++)
 #pragma unroll
         for (int di = -1; di <= 1; di++)
-#pragma unroll
-            for (int dk = -KR; dk <= KR; dk++) {
-                const bool in = ok_j[dj + 1] && ok_i[di + 1] && (DIM == 2 || ok_k[dk + 1]);
-                v[((dj + 1) * 3 + di + 1) * (2 * KR + 1) + dk + KR] = in ? (TA)base[dj * sj + di * si + dk * DIM] : TA(0);
-            }
-    TA acc = TA(0);
+            v[(dj + 1) * 3 + di + 1] = ok_j[dj + 1] && ok_i[di + 1] ? (TO)base[dj * sj + di * 2] : TO(0);
+    TO acc = TO(0);
 #pragma unroll
     for (int dj = -1; dj <= 1; dj++) {
-        TA accj = TA(0);
+        TO accj = TO(0);
 #pragma unroll
         for (int di = -1; di <= 1; di++) {
-            TA acci = TA(0);
-#pragma unroll
-            for (int dk = -KR; dk <= KR; dk++) {
-                const TA q = v[((dj + 1) * 3 + di + 1) * (2 * KR + 1) + dk + KR];
-                acci += dk == 0 ? q : TA(0.5) * q;
-            }
-            accj += di == 0 ? acci : TA(0.5) * acci;
+            const TO q = v[(dj + 1) * 3 + di + 1];
+            accj += di == 0 ? q : TO(0.5) * q;
         }
-        acc += dj == 0 ? accj : TA(0.5) * accj;
+        acc += dj == 0 ? accj : TO(0.5) * accj;
     }
     if (done) return;
-    const TO bc = (TO)(acc * ti * tj * tk);
-    vc[c * DIM + d] = bc;
+    const TO bc = (TO)(acc * ti * tj);
+    vc[t] = bc;
     // first smoothing sweep of the coarse level from x = 0: x = omega * scale / diag * b
-    if (j0.x) j0.x[c * DIM + d] = jw * bc;
+    if (j0.x) j0.x[t] = jw * bc;
+}
+
+// 3D restriction by rows: the block of coarse rows (ic0 .. ic0 + NI - 1, jc), or of a chunk of KCB <=
+// kRestrictKC coarse nodes of them along z.  Thread s takes component s % 3 of fine node s / 3 along
+// z, in the 3 x (2 NI + 1) fine rows that those coarse rows read: loads consecutive across the warp,
+// the x and y stages in registers; the z stage goes through shared memory, where the two threads of a
+// coarse node share its NI rows.  Per axis the weights are 0.5 / 1 / 0.5 and 1/tw factorises into
+// 1/1.5 (boundary node) or 1/2.
+// Bound by the loads on the fine levels and by latency on the others.  One thread per coarse value
+// reading its 27 fine ones every other node took 2.06 us from 24x12x12 (now 1.55) and 12.6 us from
+// 192x96x96 (11.3) in FP64, and 25.7 us of the 256x128x128 FP32 V-cycle, now 6 us less.  Blocks of
+// up to 256 threads: with whole rows of 416 only one fits an SM beside the 27 loads in flight (FP64
+// 45 us from 256x128x128 instead of 35).
+constexpr int kRestrictKC = 42;
+template <int NI, typename TI, typename TO>
+__global__ void __launch_bounds__((6 * kRestrictKC + 3 + 31) / 32 * 32) k_restrict_rows(GridDev<3> gf, GridDev<3> gc, int chunks, int KCB, const TI* __restrict__ vf,
+                                                       TO* __restrict__ vc, const int* skip, Jacobi0<TO> j0) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ TO s_a[NI][3 * (2 * kRestrictKC + 1)];
+    const int done = skip ? *skip : 0;  // looked at only once the values are on their way
+    const unsigned row = blockIdx.x / (unsigned)chunks;
+    const int kc0 = (int)(blockIdx.x - row * (unsigned)chunks) * KCB;
+    const int nxb = (gc.nn[0] + NI - 1) / NI;
+    const int jc = (int)(row / (unsigned)nxb), ic0 = (int)(row - (unsigned)jc * (unsigned)nxb) * NI;
+    const int s = (int)threadIdx.x, f = s / 3, d = s - 3 * f;
+    const int KC = min(KCB, gc.nn[2] - kc0);  // coarse nodes of this block
+    const int k = 2 * kc0 - 1 + f;                    // fine node
+    const bool in_k = f <= 2 * KC && k >= 0 && k < gf.nn[2];
+    // values outside the grid are not read but their place in the sums is kept
+    TO v[3][2 * NI + 1];
+    const int si = gf.nn[2] * 3;
+    const long long sj = (long long)si * gf.nn[0];
+    const TI* base = vf + (2 * jc - 1) * sj + (long long)(2 * ic0 - 1) * si + 3 * k + d;
+#pragma unroll
+    for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int a = 0; a < 2 * NI + 1; a++) {
+            const int j = 2 * jc - 1 + b, i = 2 * ic0 - 1 + a;
+            v[b][a] = in_k && j >= 0 && j < gf.nn[1] && i >= 0 && i < gf.nn[0] ? (TO)base[b * sj + a * si] : TO(0);
+        }
+    const int q = f >> 1, kc = kc0 + q;  // this thread's coarse node: rows ic0 + (f & 1), + 2, ..
+    const bool out = q < KC;
+    const long long c0 = nidx(gc, ic0, jc, kc) * 3 + d;
+    TO jw[(NI + 1) / 2];
+#pragma unroll
+    for (int m = 0; m < (NI + 1) / 2; m++) {
+        const int a = 2 * m + (f & 1);
+        jw[m] = TO(0);
+        if (j0.x && out && a < NI && ic0 + a < gc.nn[0])
+            jw[m] = (TO)((*j0.omega) * j0.scale) * j0.dinv[c0 + (long long)a * gc.nn[2] * 3];
+    }
+    if (f <= 2 * KC) {
+#pragma unroll
+        for (int a = 0; a < NI; a++) {
+            TO y[3];
+#pragma unroll
+            for (int b = 0; b < 3; b++) y[b] = v[b][2 * a + 1] + TO(0.5) * (v[b][2 * a] + v[b][2 * a + 2]);
+            s_a[a][s] = y[1] + TO(0.5) * (y[0] + y[2]);
+        }
+    }
+    __syncthreads();
+    if (done || !out) return;
+    auto itw = [](int c, int n) { return (c == 0 || c == n - 1) ? TO(1.0 / 1.5) : TO(0.5); };
+    const TO tjk = itw(jc, gc.nn[1]) * itw(kc, gc.nn[2]);
+#pragma unroll
+    for (int m = 0; m < (NI + 1) / 2; m++) {
+        const int a = 2 * m + (f & 1);
+        if (a >= NI || ic0 + a >= gc.nn[0]) continue;
+        const TO* z = s_a[a] + 6 * q + d;
+        const TO bc = (z[3] + TO(0.5) * (z[0] + z[6])) * (tjk * itw(ic0 + a, gc.nn[0]));
+        const long long c = c0 + (long long)a * gc.nn[2] * 3;
+        vc[c] = bc;
+        // first smoothing sweep of the coarse level from x = 0: x = omega * scale / diag * b
+        if (j0.x) j0.x[c] = jw[m] * bc;
+    }
 }
 
 // One thread per fine node (all DIM components, contiguous loads of each parent): P =
@@ -239,10 +301,17 @@ int launch_restrict(const Grid& gf, const TI* vf, TO* vc, const int* skip, cudaS
     const Grid gc = coarse_grid(gf);
     const unsigned nb = (unsigned)((gc.n_nodes * gf.dim + 255) / 256);
     pf::count_launch();
-    if (gf.dim == 3)
-        PF_CUDA(launch_pdl(k_restrict<3, TI, TO>, dim3(nb), dim3(256), 0, st, gdev<3>(gf), gdev<3>(gc), vf, vc, skip, j0));
-    else
-        PF_CUDA(launch_pdl(k_restrict<2, TI, TO>, dim3(nb), dim3(256), 0, st, gdev<2>(gf), gdev<2>(gc), vf, vc, skip, j0));
+    if (gf.dim == 3) {
+        const int chunks = (gc.nn[2] + kRestrictKC - 1) / kRestrictKC;
+        const int kc = (gc.nn[2] + chunks - 1) / chunks, th = (3 * (2 * kc + 1) + 31) / 32 * 32;
+        // four rows per thread once that still gives every SM three blocks (from 128x64x64 FP64 5.2 us;
+        // one row 6.2; from 96x48x48 3.4 against 3.7 the other way round)
+        const bool four = (long long)((gc.nn[0] + 3) / 4) * gc.nn[1] * chunks >= 3LL * kNumSM;
+        const long long rows = (long long)(four ? (gc.nn[0] + 3) / 4 : gc.nn[0]) * gc.nn[1];
+        PF_CUDA(launch_pdl(four ? k_restrict_rows<4, TI, TO> : k_restrict_rows<1, TI, TO>, dim3((unsigned)(rows * chunks)),
+                           dim3(th), 0, st, gdev<3>(gf), gdev<3>(gc), chunks, kc, vf, vc, skip, j0));
+    } else
+        PF_CUDA(launch_pdl(k_restrict_q<TI, TO>, dim3(nb), dim3(256), 0, st, gdev<2>(gf), gdev<2>(gc), vf, vc, skip, j0));
     PF_LAUNCH_CHECK("restrict launch");
     return PF_OK;
 }

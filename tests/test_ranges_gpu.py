@@ -251,3 +251,14 @@ def test_coarse_inverse(lib, nel, n_level):
     r[wl["fixed_dofs"]] = 0.0
     z = N(s.vcycle(T(r), omega=0.4))
     assert rel(z, O.mg_vcycle(nel, unit_K0(dim), E, wl["fixed_dofs"], r, n_level=n_level, omega=0.4)) < 1e-9
+
+
+@pytest.mark.parametrize("nel", [
+    (2, 2, 2), (2, 3, 5), (7, 5, 82), (6, 4, 84), (5, 9, 169), (300, 62, 10), (301, 63, 85), (2, 600, 600), (31, 18)])
+def test_restriction_rows(lib, nel):
+    # 27 products and sums per value on each side, each within 1.1e-16 of the sum of magnitudes
+    vf = np.random.default_rng(5).standard_normal(O.n_nodes(nel) * len(nel))
+    grid, vft = lib.make_grid(nel), T(vf)
+    out = torch.full((O.n_nodes(O.coarse_nel(nel)) * len(nel),), np.nan, dtype=torch.float64, device="cuda")
+    lib.check(lib.load().pf_restrict_f64(ctypes.byref(grid), lib.ptr(vft), lib.ptr(out), lib.stream()))
+    assert np.all(np.abs(N(out) - O.restrict(nel, vf)) <= 60 * 1.2e-16 * O.restrict(nel, np.abs(vf)))
