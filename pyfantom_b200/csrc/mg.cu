@@ -79,6 +79,7 @@ struct pf_mg {
     uint8_t* node_flag = nullptr;
     const double* E = nullptr;
     const uint8_t* mask = nullptr;
+    bool bottom = false;            // last smoothed level and dense solve in one launch
     pf::CoarseOp* c1 = nullptr;     // element-level operator of level 1 (else its stencil)
     // deflation by a coarse space Q = [q_0 q_1 q_2], q_c = a field's component c (learned
     // coarse-grid correction): field, W = A Q (FP32) and G^-1 (FP64, 9 values + 3 flags)
@@ -582,6 +583,10 @@ static int vcycle(pf_mg* mg, int l, const T* b0, T** res, double* dot_partials, 
     T* X = (T*)L.x;
     T* Tb = (T*)L.t;
     int s;
+    if (l == mg->nlev - 1 && x_ready && mg->bottom) {
+        *res = Tb;
+        return launch_bottom<T>(L.g, (const T*)L.H, b, (const T*)X, dinv, Tb, &mg->dense, mg->cfg.n_smooth, omega, scale, skip, st);
+    }
     if (!x_ready) {  // otherwise the restriction from the finer level did this sweep
         pf::count_launch();
         PF_CUDA(launch_pdl(k_jacobi0<T>, dim3(vec_blocks(L.ndof)), dim3(kRedThreads), 0, st, L.ndof, b, dinv, omega, scale, X, skip));
@@ -751,6 +756,10 @@ extern "C" int pf_mg_create(const pf_op* op, const pf_mg_config* cfg, pf_mg** ou
     if (!s && ncoarse > 6144)
         s = fail(PF_BAD_ARG, "coarsest level has %lld DOF (> 6144): use more levels", ncoarse);
     if (!s) s = dense_alloc(&mg->dense, (int)ncoarse);
+    // a stencil level below the fine one, visited once per cycle
+    const int lb = mg->nlev - 1;
+    if (!s && lb >= 1 && mg->L[lb].H && !(lb < 32 && ((cfg->w_mask >> lb) & 1u)))
+        mg->bottom = mg->fp32 ? bottom_fits<float>(mg->L[lb].g) : bottom_fits<double>(mg->L[lb].g);
     const int nc = g.dim == 3 ? 8 : 4, nd = nc * g.dim;
     s = s ? s : dalloc((void**)&mg->K0_dev, nd * nd * sizeof(double));
     s = s ? s : dalloc((void**)&mg->Kc_dev, (size_t)nc * nd * nd * sizeof(double));

@@ -340,6 +340,307 @@ template int launch_prolong<double>(const Grid&, const double*, double*, const i
 template int launch_prolong<float>(const Grid&, const float*, float*, const int*, cudaStream_t);
 
 // ---------------------------------------------------------------------------------------
+// bottom of the V-cycle: the last smoothed level and the dense solve below it in one launch
+// ---------------------------------------------------------------------------------------
+// A cluster of kBottomCTAs blocks.  Block r owns nodes [r npc, (r + 1) npc); thread (node n, group
+// grp < 9) keeps the 27 stencil values of offsets 3 grp .. 3 grp + 2 in registers through the
+// 2 n_smooth products.  A product's result is stored into every block's copy of the level vector, so
+// that one cluster barrier separates two steps; the restricted residual and the prolonged correction
+// are formed by every block for itself.
+// Bound by latency: 13x7x7 nodes over 336 coarse values, n_smooth 2, FP64: 2 us to read the operators
+// (beside the launch before), 1.4 to 2.3 us per product, of which 1 us for its distribution and the
+// barrier, 2.1 us for the coarse inverse.  Level by level it was seven launches and 16 us: FP64
+// V-cycle of 96x48x48 140.8 -> 133.5 us, mixed of 192x96x96 352.8 -> 339.2 us.  With the stencil in
+// shared memory and read again for each product, and the inverse read from L2, it was 36 us.
+constexpr int kBottomCTAs = 16;
+
+template <typename T>
+struct BottomArgs {
+    GridDev<3> g, gc;
+    const T* H;  // half storage of the level's stencil
+    const T *b, *x0, *dinv;
+    T* out;
+    const double* Ainv;
+    int np, ns, npc;
+    int inv_off, inv_rows;  // rows of Ainv held in shared memory (per block), at this byte offset
+    const double* omega;
+    double scale;
+    const int* skip;
+};
+
+template <typename T>
+struct BottomSmem {  // offsets in values of T
+    int u, b, d, x, r, part, bc, xc, end;
+    __host__ __device__ BottomSmem(int npc, int N, int Nc) {
+        u = 0, b = 6 * N, d = b + 3 * npc, x = d + 3 * npc, r = x + 3 * npc, part = r + 3 * npc;
+        bc = part + 27 * npc, xc = bc + 3 * Nc, end = xc + 3 * Nc;
+    }
+};
+
+template <typename T>
+__device__ __forceinline__ void st_rank(T* p, int rank, T v) {  // *p of block `rank`
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    if constexpr (sizeof(T) == 8)
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+    else
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, 1) k_mg_bottom(const BottomArgs<T> p) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int N = (int)p.g.n_nodes, Nc = (int)p.gc.n_nodes, npc = p.npc, rank = blockIdx.x, tid = threadIdx.x;
+    cluster_arrive();  // every block has started: before the first store into another one
+    const BottomSmem<T> so(npc, N, Nc);
+    T* const sm = reinterpret_cast<T*>(s_raw);
+    T *const sb = sm + so.b, *const sd = sm + so.d, *const sx = sm + so.x, *const sr = sm + so.r;
+    T *const part = sm + so.part, *const sbc = sm + so.bc, *const sxc = sm + so.xc;
+    const int n0 = rank * npc, nloc = max(0, min(npc, N - n0));
+    const int sj = p.g.nn[2] * p.g.nn[0], si = p.g.nn[2];
+    // The stencil and the coarse inverse are written by the setup, several launches back: they are
+    // read (the inverse into L2) while the launch before this one still runs.
+    const int grp = (unsigned)tid / (unsigned)npc, n = tid - grp * npc;
+    const bool item = grp < 9 && n < nloc;
+    T A[27];
+    int m[3];  // the neighbours' places in a level vector
+    {
+        int i = 0, j = 0, k = 0;
+        if (item) ndec(p.g, n0 + n, i, j, k);
+        const int oy = grp % 3 - 1, oz = grp / 3 - 1;
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const bool ok = item && nok(p.g, i + q - 1, j + oy, k + oz);
+            m[q] = 3 * (ok ? n0 + n + oz + (q - 1) * si + oy * sj : item ? n0 + n : 0);
+            // as in k_stencil_matvec: a lower offset is its neighbour's opposite block, transposed
+            constexpr int C = 13;
+            const int o = 3 * grp + q, t = o >= C ? n0 + n : m[q] / 3, sa = o >= C ? 96 : 32;
+            const T* Ho = p.H + ((long long)(t >> 5) * (C + 1) + abs(o - C)) * 9 * 32 + (t & 31);
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+#pragma unroll
+                for (int b = 0; b < 3; b++) A[9 * q + 3 * a + b] = ok ? __ldcg(Ho + a * sa + b * (128 - sa)) : T(0);
+        }
+    }
+    const int nrow = (3 * Nc - rank + kBottomCTAs - 1) / kBottomCTAs;  // rows rank, rank + kBottomCTAs, ..
+    double* const s_inv = reinterpret_cast<double*>(s_raw + p.inv_off);
+    const int c2 = (3 * Nc + 1) / 2, ld = 2 * c2;  // pairs per row; a row is padded to pairs (np is even)
+    for (int t = tid; t < min(nrow, p.inv_rows) * c2; t += NT) {
+        const int r = (unsigned)t / (unsigned)c2, c = 2 * (t - r * c2);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(s_inv + r * ld + c)),
+                     "l"(p.Ainv + (long long)(rank + r * kBottomCTAs) * p.np + c)
+                     : "memory");
+    }
+    pdl_wait();
+    pdl_trigger();
+    const int done = p.skip ? *p.skip : 0;  // the same for all blocks
+    const T w = (T)((*p.omega) * p.scale);
+    T* u = sm + so.u;  // the current level vector (all nodes)
+    T* v = u + 3 * N;  // the next one
+#pragma unroll 4
+    for (int t = tid; t < 3 * N; t += NT) u[t] = p.x0[t];
+    for (int t = tid; t < 3 * nloc; t += NT) {
+        sb[t] = p.b[3 * n0 + t];
+        sd[t] = p.dinv[3 * n0 + t];
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    cluster_wait();
+    if (done) return;
+    __syncthreads();
+    // f(own DOF, (A u) there)
+    auto product = [&](auto f) {
+        if (item) {
+            T acc[3] = {T(0), T(0), T(0)};
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const T u0 = u[m[q]], u1 = u[m[q] + 1], u2 = u[m[q] + 2];
+#pragma unroll
+                for (int a = 0; a < 3; a++)
+                    acc[a] = fma(A[9 * q + 3 * a], u0, fma(A[9 * q + 3 * a + 1], u1, fma(A[9 * q + 3 * a + 2], u2, acc[a])));
+            }
+#pragma unroll
+            for (int a = 0; a < 3; a++) part[(grp * npc + n) * 3 + a] = acc[a];
+        }
+        __syncthreads();
+        if (tid < 3 * nloc) {
+            T y = part[tid];
+#pragma unroll
+            for (int q = 1; q < 9; q++) y += part[q * 3 * npc + tid];
+            f(tid, y);
+        }
+    };
+    auto share = [&](int t, T val) {
+#pragma unroll
+        for (int r = 0; r < kBottomCTAs; r++) st_rank(v + 3 * n0 + t, r, val);
+    };
+    auto next = [&]() {  // everybody's values are in v
+        cluster_arrive();
+        cluster_wait();
+        T* q = u;
+        u = v;
+        v = q;
+    };
+    for (int k = 1; k < p.ns; k++) {
+        product([&](int t, T y) { share(t, u[3 * n0 + t] + w * sd[t] * (sb[t] - y)); });
+        next();
+    }
+    product([&](int t, T y) {
+        sx[t] = u[3 * n0 + t];
+        sr[t] = sb[t] - y;
+        share(t, sr[t]);
+    });
+    next();
+    // restriction (the values of k_restrict_rows)
+    auto itw = [](int c, int nn) { return (c == 0 || c == nn - 1) ? T(1.0 / 1.5) : T(0.5); };
+    for (int t = tid; t < 3 * Nc; t += NT) {
+        const int c = (unsigned)t / 3u, d = t - 3 * c;
+        int i, j, k;
+        ndec(p.gc, c, i, j, k);
+        const T* uc = u + 3 * (2 * k + si * 2 * i + sj * 2 * j) + d;
+        T acc = T(0);
+#pragma unroll
+        for (int b = -1; b <= 1; b++)
+#pragma unroll
+            for (int a = -1; a <= 1; a++)
+#pragma unroll
+                for (int q = -1; q <= 1; q++)
+                    acc += T((a ? 0.5 : 1.0) * (b ? 0.5 : 1.0) * (q ? 0.5 : 1.0)) *
+                           (nok(p.g, 2 * i + a, 2 * j + b, 2 * k + q) ? uc[3 * (q + a * si + b * sj)] : T(0));
+        sbc[t] = acc * (itw(i, p.gc.nn[0]) * itw(j, p.gc.nn[1]) * itw(k, p.gc.nn[2]));
+    }
+    __syncthreads();
+    // x_c = A_c^-1 b_c, accumulation in FP64, a row per warp; the loads of 12 x 32 columns are in
+    // flight together.  Stored divided by tw, so that the prolongation takes plain means.
+    const int l = tid & 31;
+    for (int r = tid >> 5; r < nrow; r += NT / 32) {
+        const int row = rank + r * kBottomCTAs;
+        const double* Ar = r < p.inv_rows ? s_inv + r * ld : p.Ainv + (long long)row * p.np;
+        double s = 0.0;
+        for (int c0 = l; c0 < 3 * Nc; c0 += 12 * 32) {
+            double a[12];
+#pragma unroll
+            for (int q = 0; q < 12; q++) a[q] = c0 + 32 * q < 3 * Nc ? Ar[c0 + 32 * q] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 12; q++)
+                if (c0 + 32 * q < 3 * Nc) s += a[q] * (double)sbc[c0 + 32 * q];
+        }
+        s = __shfl_sync(0xffffffffu, warp_sum(s), 0);
+        int i, j, k;
+        ndec(p.gc, row / 3, i, j, k);
+        const T x = (T)s * (itw(i, p.gc.nn[0]) * itw(j, p.gc.nn[1]) * itw(k, p.gc.nn[2]));
+        if (l < kBottomCTAs) st_rank(sxc + row, l, x);
+    }
+    cluster_arrive();
+    cluster_wait();
+    // prolongation (the values of k_prolong): the mean over the parents, one that is alone along an
+    // axis taken twice
+#pragma unroll 4
+    for (int t = tid; t < 3 * N; t += NT) {
+        const int f = (unsigned)t / 3u, d = t - 3 * f;
+        int i, j, k;
+        ndec(p.g, f, i, j, k);
+        const int ck = p.gc.nn[2], ci = p.gc.nn[0];
+        const int k1 = (k >> 1) + (k & 1) < ck ? 3 * (k & 1) : 0, i1 = (i >> 1) + (i & 1) < ci ? 3 * ck * (i & 1) : 0;
+        const int j1 = (j >> 1) + (j & 1) < p.gc.nn[1] ? 3 * ck * ci * (j & 1) : 0;
+        const T* x = sxc + 3 * ((k >> 1) + ck * ((i >> 1) + ci * (j >> 1))) + d;
+        v[t] = T(0.125) * (((x[0] + x[k1]) + (x[i1] + x[i1 + k1])) + ((x[j1] + x[j1 + k1]) + (x[j1 + i1] + x[j1 + i1 + k1])));
+    }
+    {
+        T* q = u;
+        u = v;
+        v = q;
+    }
+    __syncthreads();
+    for (int k = 1; k < p.ns; k++) {
+        product([&](int t, T y) { share(t, u[3 * n0 + t] + w * sd[t] * (sr[t] - y)); });
+        next();
+    }
+    product([&](int t, T y) { p.out[3 * n0 + t] = sx[t] + u[3 * n0 + t] + w * sd[t] * (sr[t] - y); });
+}
+
+// A level fits when the stencil goes into the cluster's registers, 27 values per thread: 512 threads
+// per block in FP64 (896 nodes), 1024 in FP32 (1808).  Only 16 SMs read the coarse inverse: 675 values
+// take 6.6 us of the kernel where a launch over all SMs takes 4, and the 256x128x128 V-cycle still
+// gained 13 us (699 -> 686); the line is drawn a little above.
+constexpr int kBottomCoarse = 768;
+
+static int bottom_npc(const Grid& g) { return (int)((g.n_nodes + kBottomCTAs - 1) / kBottomCTAs); }
+// shared memory: the vectors, then as many of the block's rows of the coarse inverse as fit
+constexpr int kBottomSmem = 200 * 1024;
+template <typename T>
+static size_t bottom_smem(const Grid& g, int* inv_off, int* inv_rows) {
+    const int nc = 3 * (int)coarse_grid(g).n_nodes, row = (nc + 1) / 2 * 16, rows = (nc + kBottomCTAs - 1) / kBottomCTAs;
+    const int off = (int)(sizeof(T) * BottomSmem<T>(bottom_npc(g), (int)g.n_nodes, nc / 3).end + 15) / 16 * 16;
+    const int fit = (kBottomSmem - off) / row;
+    *inv_off = off;
+    *inv_rows = fit < rows ? fit : rows;
+    return off + (size_t)*inv_rows * row;
+}
+template <typename T>
+static cudaLaunchConfig_t bottom_config(const Grid& g, int threads, cudaLaunchAttribute* attr, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    int off, rows;
+    cfg.gridDim = dim3(kBottomCTAs);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = bottom_smem<T>(g, &off, &rows);
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kBottomCTAs;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+template <typename T>
+static auto bottom_kernel(const Grid& g, int* threads) {
+    *threads = sizeof(T) == 8 || 9 * bottom_npc(g) <= 512 ? 512 : 1024;
+    return *threads == 512 ? k_mg_bottom<T, 512> : k_mg_bottom<T, sizeof(T) == 8 ? 512 : 1024>;
+}
+
+template <typename T>
+bool bottom_fits(const Grid& g) {
+    if (g.dim != 3 || g.n_nodes > kBottomCTAs * 113) return false;
+    int threads, n = 0;
+    auto kernel = bottom_kernel<T>(g, &threads);
+    if (9 * bottom_npc(g) > threads || coarse_grid(g).n_nodes * 3 > kBottomCoarse) return false;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = bottom_config<T>(g, threads, attr, nullptr);
+    cfg.numAttrs = 1;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBottomSmem) == cudaSuccess &&
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+    return ok;
+}
+
+template <typename T>
+int launch_bottom(const Grid& g, const T* H, const T* b, const T* x0, const T* dinv, T* out, const Dense* d, int ns,
+                  const double* omega, double scale, const int* skip, cudaStream_t st) {
+    int threads;
+    auto kernel = bottom_kernel<T>(g, &threads);
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = bottom_config<T>(g, threads, attr, st);
+    int off, rows;
+    bottom_smem<T>(g, &off, &rows);
+    const BottomArgs<T> a{gdev<3>(g), gdev<3>(coarse_grid(g)), H, b, x0, dinv, out, d->Ainv, d->np, ns, bottom_npc(g),
+                          off, rows, omega, scale, skip};
+    pf::count_launch();
+    PF_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
+    PF_LAUNCH_CHECK("V-cycle bottom launch");
+    return PF_OK;
+}
+template bool bottom_fits<double>(const Grid&);
+template bool bottom_fits<float>(const Grid&);
+template int launch_bottom<double>(const Grid&, const double*, const double*, const double*, const double*, double*, const Dense*,
+                                   int, const double*, double, const int*, cudaStream_t);
+template int launch_bottom<float>(const Grid&, const float*, const float*, const float*, const float*, float*, const Dense*,
+                                  int, const double*, double, const int*, cudaStream_t);
+
+// ---------------------------------------------------------------------------------------
 // block-stencil matvec (levels >= 1): y_n = sum_o A[n,o] u_{n+o}
 // A block covers 32 consecutive nodes; warp w gathers the neighbour offsets 3w..3w+2 for
 // all 32 nodes (coalesced reads of the structure-of-arrays coefficients), the per-warp

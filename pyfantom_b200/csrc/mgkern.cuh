@@ -65,4 +65,12 @@ int dense_factor_linv(Dense* d, double beta, cudaStream_t st);
 template <typename T>
 int dense_solve(const Dense* d, const T* b, T* x, const int* skip, cudaStream_t st);
 
+// one V-cycle of level g (3D, from the swept x0) over its dense coarse solve d in one launch, for a
+// level that fits (a property of its size and the device): out = the corrected iterate
+template <typename T>
+bool bottom_fits(const Grid& g);
+template <typename T>
+int launch_bottom(const Grid& g, const T* H, const T* b, const T* x0, const T* dinv, T* out, const Dense* d, int ns,
+                  const double* omega, double scale, const int* skip, cudaStream_t st);
+
 }  // namespace pf

@@ -262,3 +262,24 @@ def test_restriction_rows(lib, nel):
     out = torch.full((O.n_nodes(O.coarse_nel(nel)) * len(nel),), np.nan, dtype=torch.float64, device="cuda")
     lib.check(lib.load().pf_restrict_f64(ctypes.byref(grid), lib.ptr(vft), lib.ptr(out), lib.stream()))
     assert np.all(np.abs(N(out) - O.restrict(nel, vf)) <= 60 * 1.2e-16 * O.restrict(nel, np.abs(vf)))
+
+
+@pytest.mark.parametrize("nel,nl,ns,kw", [
+    ((8, 8, 8), 3, 2, {}), ((48, 24, 24), 3, 2, {}), ((24, 16, 8), 3, 1, {}), ((40, 24, 28), 3, 3, {}),
+    ((36, 28, 32), 3, 2, {}), ((20, 18, 18), 2, 2, dict(coarse_op="stencil")), ((20, 20, 20), 2, 2, dict(coarse_op="stencil"))])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_vcycle_bottom(nel, nl, ns, kw, precision):
+    # bottom levels of 27 to 1331 nodes: one launch where they fit shared memory, level by level beyond
+    from test_solver_gpu import setup_problem
+    from conftest import unit_K0
+    from pyfantom_b200 import workloads
+    wl = workloads.cantilever3d(*nel)
+    mesh, kern, sol, fe = setup_problem(wl, nl, precision=precision, n_smooth=ns, **kw)
+    kern.set_rho(T(wl["E"]))
+    sol.setup()
+    r = np.random.default_rng(0).standard_normal(kern.shape[0])
+    r[wl["fixed_dofs"]] = 0.0
+    z = N(sol.vcycle(T(r), omega=0.45))
+    zr = O.mg_vcycle(nel, unit_K0(3), wl["E"], wl["fixed_dofs"], r, n_level=nl, n_smooth=ns, omega=0.45)
+    # FP64: 2 ns products per level of conditioning below 1e5; FP32 carries 1e-7 per operation
+    assert rel(z, zr) < (1e-10 if precision == "fp64" else 1e-4)
