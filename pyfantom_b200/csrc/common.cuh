@@ -158,7 +158,19 @@ struct Epi {
     const T* dot_a;
     int dot_of_y;
     const int* skip;  // if non-NULL and *skip != 0 the kernel does nothing (solver finished)
+    double* out64 = nullptr;  // FP32 fine matvec, PF_EPI_JACOBI_ADD: written in FP64 here instead of out
 };
+
+template <typename T>
+__device__ __forceinline__ void epi_put(const Epi<T>& e, int mode, long long g, T o) {
+    if constexpr (sizeof(T) == 4) {
+        if (mode == PF_EPI_JACOBI_ADD && e.out64) {
+            e.out64[g] = (double)o;
+            return;
+        }
+    }
+    e.out[g] = o;
+}
 
 template <typename T>
 __device__ __forceinline__ T epi_apply(const Epi<T>& e, long long g, T y, T w) {

@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
                 } else if constexpr (mode == PF_EPI_JACOBI_ADD) {
                     o = pa[c] + px[c] + wgt * pd[c] * (pb[c] - y);
                 }
-                epi.out[3 * no + c] = o;
+                epi_put(epi, mode, 3 * no + c, o);
                 if constexpr (DOT) dot += (double)pt[c] * (double)(epi.dot_of_y ? y : o);
             }
         }
@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
                     } else if constexpr (mode == PF_EPI_JACOBI_ADD) {
                         o = pa[q][c] + px[q][c] + wgt * pd[q][c] * (pb[q][c] - y);
                     }
-                    epi.out[3 * no + c] = o;
+                    epi_put(epi, mode, 3 * no + c, o);
                     if constexpr (DOT) dot += (double)pt[q][c] * (double)(epi.dot_of_y ? y : o);
                 }
             }
@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(256) k_matvec_q4(int NX, int NY, const T* __re
             if (mn & (1 << c)) y[c] = u[2 * n + c];
             const long long g = 2 * n + c;
             const T o = epi_apply(epi, g, y[c], wgt);
-            epi.out[g] = o;
+            epi_put(epi, epi.mode, g, o);
             if (epi.dot_partial) dot += (double)epi.dot_a[g] * (double)(epi.dot_of_y ? y[c] : o);
         }
     }
