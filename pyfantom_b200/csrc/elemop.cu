@@ -461,13 +461,22 @@ __global__ void __launch_bounds__(NW * 32, MINB)
             g[c][1][1] = dn - d;
         }
     };
-    auto escale = [&](int ie) -> T { return (elem_ok && ie >= 0 && ie < NX) ? elem_scale<T>(E[e0 + eplane * ie]) : T(0); };
+    // Without the Jacobi vectors the scale stays in its stored type from the load to the element that
+    // uses it: a conversion beside the load waits for it there (BF16 scales, STORE at 256x128x128: 68.6 -> 61.3 us).
+    // With them that wait is hidden, and the conversion at the use costs more (V-cycle 192x96x96 324 -> 328 us).
+    using EH = std::conditional_t<need_x, T, TE>;
+    auto escale = [&](int ie) -> EH {
+        if constexpr (need_x)
+            return (elem_ok && ie >= 0 && ie < NX) ? elem_scale<T>(E[e0 + eplane * ie]) : T(0);
+        else
+            return (elem_ok && ie >= 0 && ie < NX) ? E[e0 + eplane * ie] : TE(0.f);
+    };
 
     // One step (element ie = ix0 - 1 + s).
     //   v, m0, m1: plane ie+1 (loaded one step earlier); refilled with plane ie+2
     //   e: scale of element ie; refilled with that of element ie+1 after its last use
     T carry[3][2][2];
-    auto step = [&](int s, T (&gl)[3][2][2], T (&gh)[3][2][2], T (&v)[2][3], int& m0, int& m1, T& e) {
+    auto step = [&](int s, T (&gl)[3][2][2], T (&gh)[3][2][2], T (&v)[2][3], int& m0, int& m1, EH& e) {
         const int ie = ix0 - 1 + s;
         face(v, m0, m1, gh);
         if (s < CXc) load(ie + 2, v, m0, m1);
@@ -494,9 +503,9 @@ __global__ void __launch_bounds__(NW * 32, MINB)
         };
         if constexpr (!late) fetch();
         T G[3][2][2];
-        h8_element<T, CM>(gl, gh, e, cf, vb, carry, G);
+        h8_element<T, CM>(gl, gh, elem_scale<T>(e), cf, vb, carry, G);
         if constexpr (late) fetch();
-        e = (s < CXc) ? escale(ie + 1) : T(0);
+        e = (s < CXc) ? escale(ie + 1) : EH(0.f);
         // inverse y and z stages; node (je+1, kc+1) from this lane and the next, the row je
         // part to the warp below
         T P1[3];
@@ -532,7 +541,7 @@ __global__ void __launch_bounds__(NW * 32, MINB)
     T vA[2][3];
     int mA0, mA1;
     load(ix0 - 1, vA, mA0, mA1);
-    T eA = escale(ix0 - 1);
+    EH eA = escale(ix0 - 1);
     if (done) return;
     face(vA, mA0, mA1, gA);
     load(ix0, vA, mA0, mA1);
