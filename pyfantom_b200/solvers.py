@@ -8,7 +8,7 @@
   reference's V-cycle (and its lower-case ``cycle='w'`` W-cycle, which repeats the coarse
   correction at the levels in ``w_level``; the default ``'W'`` runs V-cycles there too),
   damped-Jacobi smoother, adaptive omega schedule, Galerkin
-  hierarchy and normalised transfers; the coarse solve is a dense Cholesky on the
+  hierarchy and normalised transfers; the coarse solve is a dense inverse on the
   device instead of host CHOLMOD (every reference ``coarse_solver`` name maps to it,
   with the same ``beta = 1e-6`` shift).  Keyword-only extras: ``precision`` ('fp64',
   'mixed': FP32 V-cycle inside the FP64 CG, or 'mixed_bf16': the same with the V-cycle's
