@@ -38,7 +38,7 @@ struct PcgState {
     double tol, min_omega, d_omega;
     int it, maxiter, done, status;
     int stop_le;     // 1: stop when R <= tol (cupyx cg, plain CG); 0: R < tol (MultiGrid)
-    int xlag;        // 1: the last iteration's x += alpha p is still to come
+    int xlag;        // 1: the running iteration's x += alpha p is still to come (set by PCG_CHECK, cleared by PCG_ALPHA)
     double coef[3];  // deflation: G^-1 Q^T r (start) or G^-1 W^T z (iterations)
 };
 
@@ -278,6 +278,9 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_step(const double* partials
     pdl_trigger();
     __shared__ double s_red[kRedThreads / 32];
     const int done = step != PCG_NORMB && st->done;  // looked at once the partial sums have arrived
+    // x is complete once an iteration starts: k_pcg_p of the one before has made its update, and one that
+    // ends here (no descent, not finite) makes none
+    if (step == PCG_ALPHA && threadIdx.x == 0) st->xlag = 0;
     double s[4];
     if (dG) {
         sum_partials(partials, np, s_red, s);  // r.z and W^T z
@@ -286,10 +289,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_step(const double* partials
         sum_partials(partials, np, s_red, s1);
         s[0] = s1[0];
     }
-    if (done) {
-        if (step == PCG_ALPHA && threadIdx.x == 0) st->xlag = 0;  // the iteration after the last: x is complete
-        return;
-    }
+    if (done) return;
     if (threadIdx.x == 0) {
         if (dG) defl_coef(s + 1, dG, st);
         pcg_step(step, s[0], st);

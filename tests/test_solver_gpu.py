@@ -177,6 +177,22 @@ def test_status_breakdown_on_zero_operator():
     assert sol.last_info["status"] == "PF_BREAKDOWN"
 
 
+@pytest.mark.parametrize("solver,precision", [("cg", "fp64"), ("mg", "fp64"), ("mg", "mixed")])
+def test_breakdown_keeps_the_last_iterate(solver, precision):
+    """Eight elements of negative stiffness: a direction without descent is met some iterations on.  The
+    iterate is then the one whose residual is reported.  The recursive residual differs from the true one
+    by a few 1e-16 of the largest |K x| / |b| of the iterations, here below 1e4: 1e-9."""
+    wl = workloads.cantilever3d(16, 8, 8)
+    E = np.array(wl["E"]).reshape(16, 8, 8)
+    E[4:6, 2:4, 2:4] = -0.1
+    _, kern, sol, fe = setup_problem(wl, 2, precision=precision, solver=solver)
+    b = fe.rhs.clone()
+    x, _ = sol.solve(b, rho=torch.as_tensor(E.reshape(-1), device="cuda"), use_last=False)
+    info = sol.last_info
+    assert info["status"] == "PF_BREAKDOWN" and info["iterations"] >= 1
+    assert abs(true_res(kern, x, b) - info["residual"]) < 1e-9 * info["residual"]
+
+
 def test_bad_level_count_is_rejected():
     """Four halvings of 12x8x8 leave no element on the coarsest level."""
     from pyfantom_b200._lib import PFError
