@@ -235,7 +235,9 @@ size_t pf_oc_workspace_size(long long n); /* doubles */
  * lambda in [1e-9, 1e9] until (l2-l1)/(l2+l1) <= 1e-8 testing dg.x_new - vf <= 0,
  * x_new = max(0, max(x-move, min(1, min(x+move, ocP/lambda)))) (bounds clipped to [0,1]).
  * h_out (host, may be NULL) receives {change = ||x_new - x||_2, lambda, steps}.
- * work holds pf_oc_workspace_size(n) doubles. */
+ * work holds pf_oc_workspace_size(n) doubles.  x_new may be x, df or dg (which it then replaces) or
+ * overlap df or dg in any way; one that shares no memory with x and dg serves as scratch until it is
+ * written (175 us against 206 us at 192x96x96 elements). */
 int pf_oc_update_f64(long long n, const double* x, const double* df, const double* dg, double vf,
                      double move, double* x_new, double* work, double* h_out, void* stream);
 

@@ -685,10 +685,12 @@ int oc_update(long long n, const double* x, const double* df, const double* dg, 
     double* partials = work + n;
     OcRun* S = reinterpret_cast<OcRun*>(partials + (size_t)nb * kOcTree);
     static const OcSpine sp = oc_spine();
-    // until it is written, x_new holds the lists of undecided elements (unless it is x itself,
-    // or too short for each warp's whole share and the list's head)
+    // until it is written, x_new holds the lists of undecided elements (unless it shares memory with x or
+    // dg, which every pass reads, or is too short for each warp's whole share and the list's head)
     const long long share = 32 * ((n + (long long)nb * kRT - 1) / ((long long)nb * kRT));
-    int* lists = n < (1LL << 31) && x_new != x && share + 6 <= oc_list_room(n, nb) ? reinterpret_cast<int*>(x_new) : nullptr;
+    auto apart = [&](const double* a) { return (size_t)a + n * sizeof(double) <= (size_t)x_new || (size_t)x_new + n * sizeof(double) <= (size_t)a; };
+    const bool own = apart(x) && apart(dg);
+    int* lists = n < (1LL << 31) && own && share + 6 <= oc_list_room(n, nb) ? reinterpret_cast<int*>(x_new) : nullptr;
     PF_CUDA(cudaMemsetAsync(S, 0, sizeof(OcRun), st));
     auto passes = [&](int count, int list_passes) {
         for (int p = 0; p < count + list_passes; p++) {

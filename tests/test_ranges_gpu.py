@@ -116,6 +116,33 @@ def test_oc_sequences(lib, n, kind):
     assert np.array_equal(late, got)
 
 
+@pytest.mark.parametrize("n", [257, 4800, 300_001])
+@pytest.mark.parametrize("where", ["x", "df", "dg", "dg+1", "dg-3"])
+@pytest.mark.parametrize("entry", ["work", "noalloc"])
+def test_oc_result_over_an_operand(lib, n, where, entry):
+    # x_new in the memory of an operand; the bounds are those of the separate buffers above
+    rng = np.random.default_rng(n)
+    x, df = rng.uniform(0.05, 0.95, n), -np.exp(rng.normal(0.0, 2.0, n))
+    dg = rng.uniform(0.5, 1.5, n) / n
+    vf, move = 0.4 * dg.sum(), 0.2
+    ref, steps = O.oc_update(x, df, dg, vf, move)
+    big = torch.full((n + 8,), np.nan, dtype=torch.float64, device="cuda")
+    big[4:n + 4] = T(dg)
+    xt, ft, gt = T(x), T(df), big[4:n + 4]
+    xn = {"x": xt, "df": ft, "dg": gt, "dg+1": big[5:n + 5], "dg-3": big[1:n + 1]}[where]
+    L = lib.load()
+    out = (ctypes.c_double * 3)()
+    if entry == "work":
+        work = torch.empty(int(L.pf_oc_workspace_size(n)), dtype=torch.float64, device="cuda")
+        lib.check(L.pf_oc_update_f64(n, lib.ptr(xt), lib.ptr(ft), lib.ptr(gt), vf, move, lib.ptr(xn), lib.ptr(work), out,
+                                     lib.stream()))
+    else:
+        lib.check(L.pf_oc_update_noalloc_f64(n, lib.ptr(xt), lib.ptr(ft), lib.ptr(gt), vf, move, lib.ptr(xn), out,
+                                             lib.stream()))
+    assert int(out[2]) == steps
+    assert np.abs(N(xn) - ref).max() < 1e-9
+
+
 @pytest.mark.parametrize("shape,co,stride", [
     ((1, 1, 1, 1, 1), 1, 1), ((1, 17, 2, 16, 8), 17, 1), ((2, 57, 5, 17, 9), 65, 1), ((1, 64, 3, 33, 17), 48, 2),
     ((2, 16, 16, 32, 32), 16, 1), ((8, 8, 32, 16, 16), 16, 1), ((1, 130, 4, 5, 20), 130, 1), ((1, 33, 1, 2, 3), 20, 2),
