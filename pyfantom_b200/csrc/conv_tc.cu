@@ -564,11 +564,21 @@ __global__ void __launch_bounds__(kTcWProd + 32 * kTcIssue, 1) k_conv_tc_wgrad(C
 // dw[co, ci, t] = sum over ranges of part[range][co][ci*27 + t]; db[co] from the ones row.
 // Warp g of a block adds every eighth range for 32 outputs, then the eight sums in order (one
 // thread per output over all ranges waited on 16 rounds of loads: 35 us for 128 ranges).
-__global__ void __launch_bounds__(256) k_conv_tc_wsum(const float* __restrict__ part, int nsplit, int Cout, int Mtot,
+// An output voxel that only pads a tile has dy = 0, but for a tap that lies one voxel below it (offset 0 along
+// an axis where `pad` is set) its x is the upper face of the grid: an infinity or NaN there gave 0 * inf in a tap
+// that never meets that voxel.  Such a tap whose sum is not finite is formed again from the valid outputs
+// alone (about one multiply-add per voxel and tap; nothing of it runs on finite sums).
+struct ConvPad {
+    int x, y, z;
+};
+__global__ void __launch_bounds__(256) k_conv_tc_wsum(ConvTcArgs a, ConvPad pad, const float* __restrict__ part, int nsplit,
                                                       float* __restrict__ dw, float* __restrict__ db) {
     __shared__ float s_p[8][32];
+    __shared__ double s_red[8];
+    __shared__ unsigned s_again;
+    const int Cout = a.Cout, Mtot = 27 * a.Cin + 1;
     const int g = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const long long tot = (long long)Cout * Mtot, i = (long long)blockIdx.x * 32 + l;
+    const long long tot = (long long)Cout * Mtot, i0 = (long long)blockIdx.x * 32, i = i0 + l;
     float s = 0.f;
     if (i < tot) {
 #pragma unroll 8
@@ -576,14 +586,39 @@ __global__ void __launch_bounds__(256) k_conv_tc_wsum(const float* __restrict__ 
     }
     s_p[g][l] = s;
     __syncthreads();
-    if (g != 0 || i >= tot) return;
+    if (g == 0) {
 #pragma unroll
-    for (int q = 1; q < 8; q++) s += s_p[q][l];
-    const int co = (int)(i / Mtot), m = (int)(i - (long long)co * Mtot);
-    if (m < Mtot - 1)
-        dw[(long long)co * (Mtot - 1) + m] = s;
-    else if (db)
-        db[co] = s;
+        for (int q = 1; q < 8; q++) s += s_p[q][l];
+        const int co = (int)(i / Mtot), m = (int)(i - (long long)co * Mtot), t = m % 27;
+        if (i < tot) {
+            if (m < Mtot - 1)
+                dw[(long long)co * (Mtot - 1) + m] = s;
+            else if (db)
+                db[co] = s;
+        }
+        const bool touched = (pad.x && t / 9 == 0) || (pad.y && (t / 3) % 3 == 0) || (pad.z && t % 3 == 0);
+        const unsigned again = __ballot_sync(0xffffffffu, i < tot && m < Mtot - 1 && touched && !isfinite(s));
+        if (l == 0) s_again = again;
+    }
+    __syncthreads();
+    const long long Vi = (long long)a.X * a.Y * a.Z, Vo = (long long)a.Xo * a.Yo * a.Zo;
+    for (unsigned again = s_again; again; again &= again - 1) {
+        const long long o = i0 + __ffs(again) - 1;
+        const int co = (int)(o / Mtot), m = (int)(o - (long long)co * Mtot), ci = m / 27, t = m - 27 * ci;
+        double sum = 0.0;
+        for (long long v = threadIdx.x; v < a.N * Vo && sum == sum; v += 256) {
+            const long long n = v / Vo, q = v - n * Vo;
+            const int oz = (int)(q % a.Zo), oy = (int)(q / a.Zo % a.Yo), ox = (int)(q / a.Zo / a.Yo);
+            const int gx = a.s * ox + t / 9 - 1, gy = a.s * oy + (t / 3) % 3 - 1, gz = a.s * oz + t % 3 - 1;
+            const bool in = gx >= 0 && gy >= 0 && gz >= 0 && gx < a.X && gy < a.Y && gz < a.Z;
+            const float x = in ? a.src[(n * a.Cin + ci) * Vi + ((long long)gx * a.Y + gy) * a.Z + gz] : 0.f;
+            const float d = a.w[(n * Cout + co) * Vo + q];
+            sum += (double)(__bfloat162float(__float2bfloat16_rn(x)) * __bfloat162float(__float2bfloat16_rn(d)));
+        }
+        sum = block_sum<256>(sum, s_red);
+        if (threadIdx.x == 0) dw[(long long)co * (Mtot - 1) + m] = (float)sum;
+        __syncthreads();
+    }
 }
 
 static int tc_ncols(int NP) {
@@ -709,7 +744,6 @@ extern "C" int pf_cnn_conv3d_bwd_weight_tc(const float* x, const float* dy, int 
                     out_ext(X, stride), out_ext(Y, stride), out_ext(Z, stride)};
     const long long Ktot = (long long)N * a.Xo * a.Yo * a.Zo;
     const int nsplit = (int)((Ktot + kTcWSplit - 1) / kTcWSplit);
-    const int Mtot = 27 * Cin + 1;
     // input-channel tiles of at most 56 (7 planes and the ones: 64 rows), the largest with which
     // two buffers of a tile of two or one x planes fit
     ConvWTile t;
@@ -746,8 +780,11 @@ extern "C" int pf_cnn_conv3d_bwd_weight_tc(const float* x, const float* dy, int 
     pf::count_launch(2);
     k_conv_tc_wgrad<<<dim3((unsigned)nsplit, (unsigned)(t.ntg * t.nco), (unsigned)t.nci), kTcWProd + 32 * kTcIssue, smem, st>>>(a, t,
                                                                                                                    work);
-    const long long nt = (long long)Cout * Mtot;
-    k_conv_tc_wsum<<<(unsigned)((nt + 31) / 32), 256, 0, st>>>(work, nsplit, Cout, Mtot, dw, db);
+    const long long nt = (long long)Cout * (27 * Cin + 1);
+    // padded outputs along an axis, the first of which reads the upper face (stride 2: if its extent is even)
+    auto reach = [&](int n, int no, int tile) { return no % tile != 0 && stride * no <= n; };
+    const ConvPad pad = {reach(X, a.Xo, t.TX), reach(Y, a.Yo, 16), reach(Z, a.Zo, 8)};
+    k_conv_tc_wsum<<<(unsigned)((nt + 31) / 32), 256, 0, st>>>(a, pad, work, nsplit, dw, db);
     PF_LAUNCH_CHECK("tensor-core conv weight gradient launch");
     return PF_OK;
 }

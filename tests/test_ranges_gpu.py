@@ -176,6 +176,41 @@ def test_conv_tiles(lib, shape, co, stride):
         assert rel(N(got), N(want)) < 1e-5
 
 
+@pytest.mark.parametrize("ext,stride", [((5, 17, 9), 1), ((4, 16, 8), 1), ((3, 5, 3), 1), ((6, 18, 10), 2), ((7, 35, 21), 2),
+                                       ((2, 33, 20), 1)])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_conv_weight_gradient_of_infinities(lib, ext, stride, bad):
+    # one infinity or NaN per channel on an upper face, an edge, a corner, inside: exactly the taps that meet it
+    # with a valid output are not finite; the others as in test_conv_tiles
+    N_, ci, co = 2, 9, 17
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(N_, ci, *ext, generator=g, device="cuda").to(torch.bfloat16).to(torch.float32)
+    hi, mid = [v - 1 for v in ext], [v // 2 for v in ext]
+    for c, at in enumerate([(hi[0], mid[1], mid[2]), (mid[0], hi[1], mid[2]), (mid[0], mid[1], hi[2]), (hi[0], hi[1], mid[2]),
+                            (mid[0], hi[1], hi[2]), tuple(hi), tuple(mid)]):
+        x[1, c, at[0], at[1], at[2]] = bad
+    outs = [(v - 1) // stride + 1 for v in ext]
+    dy = torch.randn(N_, co, *outs, generator=g, device="cuda").to(torch.bfloat16).to(torch.float32)
+    xp = torch.nn.functional.pad(x.double(), (1,) * 6)
+    ref = torch.empty(co, ci, 3, 3, 3, dtype=torch.float64, device="cuda")
+    for t in range(27):
+        o = (t // 9, t // 3 % 3, t % 3)
+        xs = xp[(slice(None), slice(None), *(slice(o[a], o[a] + stride * (outs[a] - 1) + 1, stride) for a in range(3)))]
+        ref[:, :, o[0], o[1], o[2]] = (xs[:, None] * dy.double()[:, :, None]).sum(dim=(0, 3, 4, 5))
+    L, P = lib.load(), lib.ptr
+    dw, db = torch.zeros(co, ci, 3, 3, 3, device="cuda"), torch.zeros(co, device="cuda")
+    work = torch.empty(int(L.pf_cnn_conv3d_bwd_weight_tc_workspace(N_, ci, *ext, co, stride)), device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    lib.check(L.pf_cnn_conv3d_bwd_weight_tc(P(x), P(dy), N_, ci, *ext, co, stride, P(dw), P(db), P(work), P(err), lib.stream()))
+    got, want = N(dw), N(ref)
+    assert int(err.item()) == 0
+    ok = np.isfinite(want)
+    assert np.array_equal(ok, np.isfinite(got)) and 0 < ok.sum() < ok.size
+    assert np.array_equal(want[~ok], got[~ok].astype(np.float64), equal_nan=True)
+    assert np.abs(got[ok] - want[ok]).max() < 1e-5 * np.abs(want[ok]).max()
+    assert rel(N(db), N(dy.double().sum(dim=(0, 2, 3, 4)))) < 1e-5
+
+
 @pytest.mark.parametrize("nel", [(1, 1), (3, 2), (2, 9), (60, 20), (20, 60), (33, 45), (45, 45), (120, 40), (300, 5), (46, 46),
                                  (1, 1, 1), (20, 1, 1), (2, 9, 2), (3, 3, 30), (4, 3, 3), (6, 5, 5)])
 def test_direct_band(lib, nel):
