@@ -7,7 +7,9 @@
 // Long thin grids (a half bandwidth of at most 96 with the nodes numbered along the shorter
 // axis first; 2D grids up to 45 elements across) are solved by a banded Cholesky factorisation
 // in 32 x 32 tiles that works inwards from both ends, k_band_solve: the constrained DOFs are
-// kept as identity rows, the band holds the free-DOF block of K.
+// kept as identity rows, the band holds the free-DOF block of K.  Elimination along a beam
+// loses more digits than across it, so the solution is corrected once with its residual in
+// pairs of doubles.
 // Other problems assemble the free-DOF matrix dense (one thread per free row gathers its
 // entries from the row node's adjacent elements, so every entry is written by one thread in a
 // fixed order), factor it by the tiled Cholesky of the coarse solver (L L^T, inverse factor
@@ -125,6 +127,26 @@ struct BandGeom {
 };
 
 __host__ __device__ inline int band_rows(const BandGeom& g, int h) { return (h ? g.nt - g.c : g.c + g.BW); }
+// node indices at[] of position p (node position * dim + component), and its DOF
+__device__ __forceinline__ int band_dof(const BandGeom& g, int p, int (&at)[3]) {
+    int rem = p / g.dim;
+    for (int a = g.dim - 1; a >= 0; a--) {
+        at[g.ord[a]] = rem % g.nn[g.ord[a]];
+        rem /= g.nn[g.ord[a]];
+    }
+    const int node = g.dim == 3 ? at[2] + g.nn[2] * (at[0] + g.nn[0] * at[1]) : at[0] + g.nn[0] * at[1];
+    return node * g.dim + p % g.dim;
+}
+// position of component 0 of the node at m[]
+__device__ __forceinline__ int band_pos(const BandGeom& g, const int (&m)[3]) {
+    int node = 0;
+    for (int a = 0; a < g.dim; a++) node = node * g.nn[g.ord[a]] + m[g.ord[a]];
+    return node * g.dim;
+}
+// entry of a right-hand side (half 0, then half 1) that holds the solution at a position
+__device__ __forceinline__ int band_at(const BandGeom& g, int gp) {
+    return gp < (g.c + g.BW) * 32 ? gp : band_rows(g, 0) * 32 + g.nt * 32 - 1 - gp;
+}
 
 // one thread per (half, local row, neighbour node): the dim entries of that row's DOF
 template <int DIM>
@@ -146,19 +168,8 @@ __global__ void k_band_assemble(BandGeom g, Grid gr, const double* __restrict__ 
         const int i = q >> 5, d = i - (ql >> 5);
         tiles[((long long)i * (g.BW + 1) + d) * 1024 + (q & 31) * 32 + (ql & 31)] = v;
     };
-    auto dof_of = [&](int p, int (&at)[3]) {
-        const int node = p / DIM;
-        int rem = node;
-        for (int a = DIM - 1; a >= 0; a--) {
-            at[g.ord[a]] = rem % g.nn[g.ord[a]];
-            rem /= g.nn[g.ord[a]];
-        }
-        const long long nd = DIM == 3 ? (long long)at[2] + (long long)gr.nn[2] * (at[0] + (long long)gr.nn[0] * at[1])
-                                      : (long long)at[0] + (long long)gr.nn[0] * at[1];
-        return (int)(nd * DIM + p % DIM);
-    };
     int at[3] = {0, 0, 0};
-    const int dof = gp < g.ndof ? dof_of(gp, at) : -1;
+    const int dof = gp < g.ndof ? band_dof(g, gp, at) : -1;
     const bool free = dof >= 0 && dof_to_free[dof] >= 0;
     if (nb == NB / 2) rhs[h * r0 + q] = (free && !(window && h)) ? b[dof] : 0.0;
     if (!free) {
@@ -191,13 +202,11 @@ __global__ void k_band_assemble(BandGeom g, Grid gr, const double* __restrict__ 
         const double w = E[ei];
         for (int k = 0; k < DIM; k++) v[k] += w * K0[(ca * DIM + comp) * ND + cb * DIM + k];
     }
-    int node = 0;
-    for (int a = 0; a < DIM; a++) node = node * g.nn[g.ord[a]] + m[g.ord[a]];
-    const long long nd = DIM == 3 ? (long long)m[2] + (long long)gr.nn[2] * (m[0] + (long long)gr.nn[0] * m[1])
-                                  : (long long)m[0] + (long long)gr.nn[0] * m[1];
+    const int p0 = band_pos(g, m);
     for (int k = 0; k < DIM; k++) {
-        if (dof_to_free[nd * DIM + k] < 0) continue;
-        const int gc = node * DIM + k, ql = h ? g.nt * 32 - 1 - gc : gc;
+        const int gc = p0 + k;
+        if (dof_to_free[band_dof(g, gc, m)] < 0) continue;
+        const int ql = h ? g.nt * 32 - 1 - gc : gc;
         if (ql > q || ql < 0) continue;
         if (window && h && gc >= g.c * 32 && gc < (g.c + g.BW) * 32) continue;  // the window's own entries: half 0
         put(ql, v[k]);
@@ -272,11 +281,15 @@ __device__ __noinline__ void band_potrf_careful(double* D, double* L, double* ri
 // Bound by the chain over the columns: one reciprocal square root, shuffle and FMA per column
 // of the longer half, about 7,500 cycles per block column (a diagonal tile with the library's
 // branching rsqrt took 12,000).  60x20 elements (2562 DOFs, 40 block columns a half): 310 us in
-// this kernel, 449 us per solve with the host's preparation, against 10,870 us for the dense
+// this kernel, 508 us per solve with the host's preparation, against 10,870 us for the dense
 // factor and its inverse.  8 warps; per block column: warp 0 factors the diagonal tile while the
 // others finish the previous column's updates, then warp w solves the tile below by w + 1
 // (and one warp the right-hand side), then all update the next diagonal tile.
-template <int BW>
+// FACTORED: the band holds the factor, and only the two substitutions run (65 us, bound by the loads
+// of each step's tiles from L2; two steps ahead instead of one 53 us, but 324 us in the other form).
+// The correction with it: 60 problems of 24x8 to 120x40 elements, contrast up to 1e9, error of the
+// solution against long double 3.3e-12 -> 4e-16 (geometric mean; the dense form 1.9e-12), 446 -> 508 us.
+template <int BW, bool FACTORED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     k_band_solve(BandGeom g, double* __restrict__ band, double* __restrict__ rhs, double* __restrict__ win,
                  const int* __restrict__ dof_to_free, int* fail) {
@@ -375,13 +388,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
                 band_potrf_careful(D, L, s_ri[p & 1], &bad);
                 if (bad >= 0 && l == 0) {  // the failing free DOF (1-based)
                     const int gp = h ? g.nt * 32 - 1 - (p * 32 + bad) : p * 32 + bad;
-                    int at[3] = {0, 0, 0}, rem = gp / g.dim;
-                    for (int a = g.dim - 1; a >= 0; a--) {
-                        at[g.ord[a]] = rem % g.nn[g.ord[a]];
-                        rem /= g.nn[g.ord[a]];
-                    }
-                    const int nd = g.dim == 3 ? at[2] + g.nn[2] * (at[0] + g.nn[0] * at[1]) : at[0] + g.nn[0] * at[1];
-                    atomicCAS(fail, 0, gp < g.ndof ? dof_to_free[nd * g.dim + gp % g.dim] + 1 : 1);
+                    int at[3];
+                    atomicCAS(fail, 0, gp < g.ndof ? dof_to_free[band_dof(g, gp, at)] + 1 : 1);
                 }
             }
         } else if (deferred) {
@@ -432,6 +440,81 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
         fetch(p + R + 1);
         __syncthreads();
     };
+    auto cluster_sync = [&]() {
+        __threadfence();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    };
+    double tl[BW][4], li[4], zl = 0.0;  // tiles of the substitutions' next step, loaded one step ahead
+    if constexpr (FACTORED) {
+        // forward: z_p = L_pp^-1 (r_p - sum_d L_p,(p-d) z_(p-d)); warp w takes rows 4 w .. 4 w + 3, its lanes the
+        // columns
+        double* part = win + BW * R * 1024;  // half 1's share of the window, reversed order
+        auto row_sums = [&](const double (&v)[4]) {  // valid for row 4 w + ((l >> 3) & 3) of the warp
+            const bool h16 = l & 16, h8 = l & 8;
+            const double a = (h16 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+            const double c = (h16 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+            double t = (h8 ? c : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : c, 8);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            return t;
+        };
+        const int row = w * 4 + ((l >> 3) & 3);
+        auto ahead = [&](int p, int end) {
+            if (p >= end) return;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                li[q] = tiles[(long long)p * R * 1024 + (w * 4 + q) * 32 + l];
+#pragma unroll
+                for (int d = 1; d <= BW; d++)
+                    tl[d - 1][q] = p >= d ? tiles[((long long)p * R + d) * 1024 + (w * 4 + q) * 32 + l] : 0.0;
+            }
+            zl = b[p * 32 + row];
+            if (h == 0 && p >= nf) zl += __ldcg(part + BW * 32 - 1 - ((p - nf) * 32 + row));
+        };
+        auto known = [&](int p, int dmin) {  // sum over d >= dmin of this lane's column
+            double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int d = 1; d <= BW; d++)
+                if (d >= dmin && p >= d) {
+                    const double z = s_x[(p - d) % R][l];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) v[q] = fma(tl[d - 1][q], z, v[q]);
+                }
+            return row_sums(v);
+        };
+        auto forward = [&](int p, int end) {
+            const double r = zl - known(p, 1);
+            double v[4];
+            if ((l & 7) == 0) s_z[0][row] = r;
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] = li[q] * s_z[0][l];
+            ahead(p + 1, end);
+            const double z = row_sums(v);
+            if ((l & 7) == 0) s_x[p % R][row] = z, b[p * 32 + row] = z;
+            __syncthreads();
+        };
+        ahead(0, nf);
+        for (int p = 0; p < nf; p++) forward(p, nf);
+        if (h == 1) {
+            for (int i = 0; i < BW; i++) {
+                const int p = nf + i;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int d = 1; d <= BW; d++)
+                        tl[d - 1][q] = p >= d ? tiles[((long long)p * R + d) * 1024 + (w * 4 + q) * 32 + l] : 0.0;
+                const double v = known(p, i + 1);
+                if ((l & 7) == 0) part[i * 32 + row] = -v;
+            }
+        }
+        cluster_sync();
+        if (h == 0) {
+            ahead(nf, rows);
+            for (int p = nf; p < rows; p++) forward(p, rows);
+        }
+        __syncthreads();
+    } else {
     for (int i = 0; i < R; i++) {
         fetch(i);
         place(i);
@@ -452,8 +535,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
             if (tid < 32) win[BW * R * 1024 + i * 32 + tid] = s_b[(nf + i) % R][tid];
         }
     }
-    __threadfence();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
     if (h == 0) {
         constexpr int NW = BW * 32;
         for (int i = 0; i < BW; i++) {
@@ -473,9 +555,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
         __syncthreads();
         for (int p = nf; p < rows; p++) column(p, rows, p > nf);
     }
-    // back substitution: x_p = L_pp^-T (z_p - sum_d L_(p+d),p^T x_(p+d)); the tiles of the next
-    // column are loaded one step ahead
-    double tl[BW][4], li[4], zl = 0.0;
+    }  // factorisation
+    // back substitution: x_p = L_pp^-T (z_p - sum_d L_(p+d),p^T x_(p+d))
     auto ahead = [&](int p) {
         if (p < 0) return;
 #pragma unroll
@@ -526,8 +607,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
         for (int p = rows - 1; p >= nf; p--) back(p);
         for (int i = tid; i < BW * 32; i += 256) win[i] = s_x[(nf + (i >> 5)) % R][i & 31];
     }
-    __threadfence();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
     if (h == 1) {
         for (int i = tid; i < BW * 32; i += 256) s_x[(nf + (i >> 5)) % R][i & 31] = __ldcg(win + BW * 32 - 1 - i);
         ahead(nf - 1);
@@ -536,20 +616,68 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     for (int p = nf - 1; p >= 0; p--) back(p);
 }
 
-// x: free entries from the halves' solutions, constrained entries the right-hand side's
+// r = b - K x over the free DOFs for the solution x = sol, in pairs of doubles (error-free products and sums), so
+// that r is exact to its own last bits; zero for the rows that half 0 or nothing holds.  NC consecutive threads
+// share a row, one element each (one thread per row, with the positions by division, took 25 us at 60x20).
+template <int DIM>
+__global__ void __launch_bounds__(128) k_band_residual(BandGeom g, Grid gr, const double* __restrict__ E, const double* __restrict__ K0,
+                                                       const int* __restrict__ dof_to_free, const double* __restrict__ b,
+                                                       const double* __restrict__ sol, double* __restrict__ res) {
+    constexpr int NC = DIM == 3 ? 8 : 4, ND = NC * DIM;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, q = t / NC, ca = t % NC;
+    const int r0 = band_rows(g, 0) * 32, nrow = r0 + band_rows(g, 1) * 32;
+    const int gp = q < r0 ? q : g.nt * 32 - 1 - (q - r0);
+    int at[3] = {0, 0, 0};
+    const int dof = q < nrow && gp < g.ndof ? band_dof(g, gp, at) : -1;
+    const bool row = dof >= 0 && dof_to_free[dof] >= 0 && band_at(g, gp) == q;
+    auto add = [](double& h, double& l, double v, double ve) {  // (h, l) += (v, ve)
+        const double t = __dadd_rn(h, v), z = __dsub_rn(t, h);
+        l += __dadd_rn(__dsub_rn(h, __dsub_rn(t, z)), __dsub_rn(v, z)) + ve;
+        h = t;
+    };
+    double hi = row && ca == 0 ? b[dof] : 0.0, lo = 0.0;
+    const int e[3] = {at[0] - kCXd(ca), at[1] - kCYd(ca), DIM == 3 ? at[2] - kCZd(ca) : 0};  // the row node is its corner ca
+    bool in = row;
+    for (int a = 0; a < DIM; a++) in = in && e[a] >= 0 && e[a] < gr.nel[a];
+    if (in) {
+        int ps[3], m[3] = {1, 1, 1};  // a step along an axis in positions and in DOFs
+        for (int a = DIM - 1, st = DIM; a >= 0; a--) {
+            ps[g.ord[a]] = st;
+            st *= g.nn[g.ord[a]];
+        }
+        const int ds[3] = {DIM == 3 ? DIM * g.nn[2] : DIM, DIM == 3 ? DIM * g.nn[2] * g.nn[0] : DIM * g.nn[0], DIM};
+        const int comp = gp % DIM;
+        double sh = 0.0, sl = 0.0;
+        for (int cb = 0; cb < NC; cb++) {
+            m[0] = kCXd(cb) - kCXd(ca), m[1] = kCYd(cb) - kCYd(ca), m[2] = DIM == 3 ? kCZd(cb) - kCZd(ca) : 0;
+            int p0 = gp - comp, d0 = dof - comp;
+            for (int a = 0; a < DIM; a++) p0 += m[a] * ps[a], d0 += m[a] * ds[a];
+            for (int k = 0; k < DIM; k++) {
+                if (dof_to_free[d0 + k] < 0) continue;
+                const double kv = K0[(ca * DIM + comp) * ND + cb * DIM + k], xv = sol[band_at(g, p0 + k)], v = __dmul_rn(kv, xv);
+                add(sh, sl, v, fma(kv, xv, -v));
+            }
+        }
+        const double w = -E[DIM == 3 ? ((long long)e[0] * gr.nel[1] + e[1]) * gr.nel[2] + e[2] : (long long)e[0] * gr.nel[1] + e[1]];
+        const double v = __dmul_rn(w, sh);
+        add(hi, lo, v, fma(w, sh, -v) + w * sl);
+    }
+#pragma unroll
+    for (int o = 1; o < NC; o <<= 1) {
+        const double h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
+        add(hi, lo, h2, l2);
+    }
+    if (q < nrow && ca == 0) res[q] = hi + lo;
+}
+
+// x: free entries from the halves' solutions and their corrections, constrained entries the right-hand side's
 __global__ void k_band_scatter(BandGeom g, const int* __restrict__ dof_to_free, const double* __restrict__ sol,
-                               const double* b, double* x) {
+                               const double* __restrict__ cor, const double* b, double* x) {
     const int gp = blockIdx.x * blockDim.x + threadIdx.x;
     if (gp >= g.ndof) return;
-    int at[3] = {0, 0, 0}, rem = gp / g.dim;
-    for (int a = g.dim - 1; a >= 0; a--) {
-        at[g.ord[a]] = rem % g.nn[g.ord[a]];
-        rem /= g.nn[g.ord[a]];
-    }
-    const int nd = g.dim == 3 ? at[2] + g.nn[2] * (at[0] + g.nn[0] * at[1]) : at[0] + g.nn[0] * at[1];
-    const int dof = nd * g.dim + gp % g.dim;
-    const int at_sol = gp < (g.c + g.BW) * 32 ? gp : band_rows(g, 0) * 32 + g.nt * 32 - 1 - gp;
-    x[dof] = dof_to_free[dof] >= 0 ? sol[at_sol] : b[dof];
+    int at[3];
+    const int dof = band_dof(g, gp, at), i = band_at(g, gp);
+    x[dof] = dof_to_free[dof] >= 0 ? sol[i] + cor[i] : b[dof];
 }
 
 // band geometry of a grid; false where the dense solve serves (bandwidth, or a grid that is
@@ -588,18 +716,18 @@ static int band_solve(pf_direct* d, const BandGeom& g, const double* E, const in
     const Grid& gr = d->op->grid;
     const long long brows = band_rows(g, 0) + band_rows(g, 1), R = g.BW + 1;
     const long long nt = brows * R * 1024;
-    const long long nwin = (g.BW * R * 1024 + g.BW * 32);
+    const long long nwin = (g.BW * R * 1024 + g.BW * 32), nrhs = brows * 32;
     // the geometry is the grid's: one allocation for the object's life
-    if (!d->band && cudaMalloc(&d->band, sizeof(double) * (nt + brows * 32 + nwin + 1)) != cudaSuccess) {
+    if (!d->band && cudaMalloc(&d->band, sizeof(double) * (nt + 2 * nrhs + nwin + 1)) != cudaSuccess) {
         cudaGetLastError();
         d->band = nullptr;
         return fail(PF_NO_MEMORY, "pf_direct_solve_f64: allocation failed");
     }
-    d->fail = reinterpret_cast<int*>(d->band + nt + brows * 32 + nwin);
-    double *rhs = d->band + nt, *win = rhs + brows * 32;
+    d->fail = reinterpret_cast<int*>(d->band + nt + 2 * nrhs + nwin);
+    double *rhs = d->band + nt, *cor = rhs + nrhs, *win = cor + nrhs;
     PF_CUDA(cudaMemsetAsync(d->band, 0, sizeof(double) * nt, st));
     PF_CUDA(cudaMemsetAsync(d->fail, 0, sizeof(int), st));
-    count_launch(3);
+    count_launch(5);
     const int nb = gr.dim == 3 ? 27 : 9;
     const unsigned blocks = (unsigned)((brows * 32 * nb + 255) / 256);
     if (gr.dim == 3)
@@ -607,16 +735,26 @@ static int band_solve(pf_direct* d, const BandGeom& g, const double* E, const in
     else
         k_band_assemble<2><<<blocks, 256, 0, st>>>(g, gr, E, d->K0, dof_to_free, b, d->band, rhs);
     PF_LAUNCH_CHECK("band assembly launch");
-    const size_t sm = (size_t)R * R * kBTile * sizeof(double);
-    auto solve = [&](auto kernel) {
-        PF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kernel<<<2, 256, sm, st>>>(g, d->band, rhs, win, dof_to_free, d->fail);
+    auto solve = [&](auto kernel, size_t sm, double* v) {
+        if (sm) PF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        kernel<<<2, 256, sm, st>>>(g, d->band, v, win, dof_to_free, d->fail);
         PF_LAUNCH_CHECK("band solve launch");
         return (int)PF_OK;
     };
-    const int s = g.BW == 1 ? solve(k_band_solve<1>) : g.BW == 2 ? solve(k_band_solve<2>) : solve(k_band_solve<3>);
+    const size_t sm = (size_t)R * R * kBTile * sizeof(double);
+    int s = g.BW == 1 ? solve(k_band_solve<1, false>, sm, rhs)
+          : g.BW == 2 ? solve(k_band_solve<2, false>, sm, rhs) : solve(k_band_solve<3, false>, sm, rhs);
     if (s) return s;
-    k_band_scatter<<<(unsigned)((g.ndof + 255) / 256), 256, 0, st>>>(g, dof_to_free, rhs, b, x);
+    const unsigned rblocks = (unsigned)((nrhs * (gr.dim == 3 ? 8 : 4) + 127) / 128);
+    if (gr.dim == 3)
+        k_band_residual<3><<<rblocks, 128, 0, st>>>(g, gr, E, d->K0, dof_to_free, b, rhs, cor);
+    else
+        k_band_residual<2><<<rblocks, 128, 0, st>>>(g, gr, E, d->K0, dof_to_free, b, rhs, cor);
+    PF_LAUNCH_CHECK("band residual launch");
+    s = g.BW == 1 ? solve(k_band_solve<1, true>, 0, cor)
+      : g.BW == 2 ? solve(k_band_solve<2, true>, 0, cor) : solve(k_band_solve<3, true>, 0, cor);
+    if (s) return s;
+    k_band_scatter<<<(unsigned)((g.ndof + 255) / 256), 256, 0, st>>>(g, dof_to_free, rhs, cor, b, x);
     PF_LAUNCH_CHECK("direct solve launch");
     return PF_OK;
 }

@@ -2,6 +2,7 @@
 against the oracle.  Tolerances: a sum of n terms of one sign carries at most about
 n * 1.1e-16 relative error (n <= 1000 taps: 1e-13)."""
 import ctypes
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -253,6 +254,55 @@ def test_direct_band(lib, nel):
     Et[: len(E) // 2 + 1] = -1.0
     assert L.pf_direct_solve_f64(d, lib.ptr(Et), lib.ptr(ft), lib.ptr(dt), len(free), lib.ptr(bt), lib.ptr(x),
                                  lib.stream()) == lib.PF_FACTOR_FAILED
+    L.pf_direct_destroy(d)
+    L.pf_op_destroy(op)
+
+
+@pytest.mark.parametrize("nel", [(60, 20), (80, 10), (20, 45), (24, 8), (2, 1), (30, 3, 3), (4, 3, 12)])
+def test_direct_band_error(lib, nel):
+    # against the exact solution (residuals in integers): the first solve is off by cond(K) (below 1e7) times a few 1e-16,
+    # below 1e-9; the correction leaves its square and a few roundings of the result
+    from conftest import unit_K0
+    dim, K0 = len(nel), unit_K0(len(nel))
+    nn = [v + 1 for v in nel]
+    ndof = int(np.prod(nn)) * dim
+    rng = np.random.default_rng(7)
+    E = rng.uniform(0.05, 1.0, int(np.prod(nel)))
+    at = np.stack([v.reshape(-1) for v in np.meshgrid(*[np.arange(v) for v in nel], indexing="ij")], 1)
+    corners = np.array([(0, 0, 0), (1, 0, 0), (1, 1, 0), (0, 1, 0), (0, 0, 1), (1, 0, 1), (1, 1, 1), (0, 1, 1)])[:2 ** dim, :dim]
+    q = at[:, None] + corners
+    node = q[..., 0] + nn[0] * q[..., 1] if dim == 2 else q[..., 2] + nn[2] * (q[..., 0] + nn[0] * q[..., 1])
+    dofs = (node[..., None] * dim + np.arange(dim)).reshape(len(E), -1)
+    ix = (np.arange(ndof) // dim // (nn[2] if dim == 3 else 1)) % nn[0]
+    cons = np.nonzero(ix == 0)[0]
+    free = np.nonzero(ix != 0)[0].astype(np.int32)
+    b = np.zeros(ndof)
+    b[ix == nel[0]] = -1.0
+    A = np.zeros((ndof, ndof))
+    np.add.at(A, (dofs[:, :, None], dofs[:, None, :]), E[:, None, None] * K0)
+    inv = np.linalg.inv(A[np.ix_(free, free)])
+    fix = np.vectorize(lambda v, bits: int(Fraction(float(v)) * 2 ** bits), otypes=[object])  # exact: no bit is cut off
+    Ke = fix(E, 70)[:, None, None] * fix(K0, 130)
+    assert np.all(Ke.astype(np.float64) * 2.0 ** -200 == E[:, None, None] * K0)
+    x100, b300 = np.zeros(ndof, dtype=object), fix(b, 300)  # x in units of 2^-100
+    for _ in range(12):
+        y = np.zeros(ndof, dtype=object)
+        np.add.at(y, dofs, (Ke * x100[dofs][:, None, :]).sum(axis=-1))
+        step = inv @ ((b300 - y)[free].astype(np.float64) * 2.0 ** -300)
+        x100[free] += fix(step, 100)
+    ref = x100.astype(np.float64) * 2.0 ** -100
+    assert np.abs(step).max() < 1e-20 * np.abs(ref).max()
+    d2f = np.full(ndof, -1, dtype=np.int32)
+    d2f[free] = np.arange(len(free), dtype=np.int32)
+    L = lib.load()
+    grid, op, d = lib.make_grid(nel), ctypes.c_void_p(), ctypes.c_void_p()
+    K0c = np.ascontiguousarray(K0)
+    lib.check(L.pf_op_create(ctypes.byref(grid), K0c.ctypes.data, ctypes.byref(op)))
+    lib.check(L.pf_direct_create(op, ctypes.byref(d)))
+    Et, ft, dt, x = T(E), T(free, torch.int32), T(d2f, torch.int32), T(b)
+    lib.check(L.pf_direct_solve_f64(d, lib.ptr(Et), lib.ptr(ft), lib.ptr(dt), len(free), lib.ptr(x), lib.ptr(x), lib.stream()))
+    assert float(np.abs((N(x) - ref)[free]).max() / np.abs(ref).max()) < 1e-15
+    assert np.array_equal(N(x)[cons], b[cons])
     L.pf_direct_destroy(d)
     L.pf_op_destroy(op)
 
