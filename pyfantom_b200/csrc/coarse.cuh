@@ -27,7 +27,7 @@ int coarse_factorise(const Op* op, double* coef);
 int coarse_create(const Op* op, int fp32, CoarseOp** out);
 void coarse_destroy(CoarseOp* c);
 // Ehat for E and the rows of the constrained elements' corners from the level-1 stencil A64;
-// *realloc set when their storage moved
+// *realloc set when their storage moved, or when the first such node came or the last one went
 int coarse_setup(CoarseOp* c, const double* E, const uint8_t* mask, const uint8_t* elem_flag, const double* A64,
                  cudaStream_t st, bool* realloc);
 template <typename T>

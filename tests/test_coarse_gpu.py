@@ -142,6 +142,27 @@ def test_level1_repeated_setup_and_growing_dirty_set():
         assert rel(U.cpu().numpy(), xo) < 1e-8
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_level1_constraints_that_come_back(precision):
+    """The captured iterations of a solve without constraints (the same mask, empty) are not used again once
+    constraints are set whose rows fit the storage of an earlier setup: iterations as with a new solver."""
+    nel = (16, 8, 8)
+    wl = workloads.cantilever3d(*nel)
+    sol, kern = _solver(nel, wl["E"], wl["fixed_dofs"], 2, precision=precision)
+    rhs, E = torch.as_tensor(wl["rhs"], device="cuda"), torch.as_tensor(wl["E"], device="cuda")
+    kern.set_constraints([])
+    sol.maxiter = 2
+    sol.solve(rhs, rho=E, use_last=False)
+    kern.set_constraints(torch.as_tensor(wl["fixed_dofs"], device="cuda"))
+    sol.maxiter = 200
+    x, _ = sol.solve(rhs, rho=E, use_last=False)
+    new, _ = _solver(nel, wl["E"], wl["fixed_dofs"], 2, precision=precision)
+    y, _ = new.solve(rhs, rho=E, use_last=False)
+    assert sol.last_info["status"] == new.last_info["status"] == "PF_OK"
+    assert sol.last_info["iterations"] == new.last_info["iterations"]
+    assert torch.equal(x, y)
+
+
 CX = [0, 1, 1, 0, 0, 1, 1, 0]
 CY = [0, 0, 1, 1, 0, 0, 1, 1]
 CZ = [0, 0, 0, 0, 1, 1, 1, 1]
