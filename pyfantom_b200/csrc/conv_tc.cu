@@ -185,7 +185,7 @@ __device__ __forceinline__ int tc_zpos(int r, int even) { return even ? (r & 1 ?
 
 // 8 values at p, p + stride, ... as BF16 (zeros where !in; the first `cnt` of them): the loads
 // are unconditional (an excluded voxel reads a valid address), so that all are in flight together
-__device__ __forceinline__ uint4 tc_gather8(const float* __restrict__ p, int stride, bool in, int cnt) {
+__device__ __forceinline__ uint4 tc_gather8(const float* __restrict__ p, long long stride, bool in, int cnt) {
     float v[8];
     if (cnt >= 8) {
 #pragma unroll
@@ -195,7 +195,7 @@ __device__ __forceinline__ uint4 tc_gather8(const float* __restrict__ p, int str
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = j < cnt ? __ldg(p + (long long)j * stride) : 0.f;
+        for (int j = 0; j < 8; j++) v[j] = j < cnt ? __ldg(p + j * stride) : 0.f;
     }
     uint4 q;
     q.x = in ? pack_bf16(v[0], v[1]) : 0u;
@@ -261,14 +261,17 @@ __global__ void __launch_bounds__(kTcProd + 32 * kTcIssue, 2) k_conv_tc(ConvTcAr
         }
         s_ntap = k;
     }
-    if (tid < kTcProd) {  // source offset of every staged voxel (-1 outside)
+    // first voxel of the tile inside the source; staged voxels by their offset from it (a source may hold more
+    // than 2^31 voxels)
+    const int g0x = max(q0x * t.step + t.org, 0), g0y = max(q0y * t.step + t.org, 0), g0z = max(q0z * t.step + t.org, 0);
+    if (tid < kTcProd) {  // offset of every staged voxel (-1 outside)
         for (int v = tid; v < nvox; v += kTcProd) {
             const int row = v / t.LZ, lx = row / t.LY;
             const int p = v - row * t.LZ, ly = row - lx * t.LY;
             const int lz = t.even ? (p < t.even ? 2 * p : 2 * (p - t.even) + 1) : p;
             const int gx = q0x * t.step + t.org + lx, gy = q0y * t.step + t.org + ly, gz = q0z * t.step + t.org + lz;
             const bool in = gx >= 0 && gy >= 0 && gz >= 0 && gx < t.SX && gy < t.SY && gz < t.SZ;
-            s_off[v] = in ? (gx * t.SY + gy) * t.SZ + gz : -1;
+            s_off[v] = in ? ((gx - g0x) * t.SY + gy - g0y) * t.SZ + gz - g0z : -1;
         }
     }
     tc_fence_before();
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(kTcProd + 32 * kTcIssue, 2) k_conv_tc(ConvTcAr
     bool ok = true;
     if (warp < 8) {
         const long long V = (long long)t.SX * t.SY * t.SZ;
-        const float* src = a.src + (long long)n * KCH * V;
+        const float* src = a.src + (long long)n * KCH * V + ((long long)g0x * t.SY + g0y) * t.SZ + g0z;
         for (int c = 0; c < nchunk; c++) {
             const int b = c & 1;
             if (c >= 2 && !mbar_wait(&s_empty[b], ((c >> 1) - 1) & 1)) ok = false;
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(kTcProd + 32 * kTcIssue, 2) k_conv_tc(ConvTcAr
 #pragma unroll 2
                 for (int v = tid; v < nvox; v += kTcProd) {
                     const int off = s_off[v];
-                    dA[h * nvox + v] = tc_gather8(sc + max(off, 0), (int)V, off >= 0, cnt);
+                    dA[h * nvox + v] = tc_gather8(sc + max(off, 0), V, off >= 0, cnt);
                 }
             }
             // weights of the chunk, lanes over the taps: (tap, half, column) -> 8 reduction channels
@@ -447,6 +450,8 @@ __global__ void __launch_bounds__(kTcWProd + 32 * kTcIssue, 1) k_conv_tc_wgrad(C
             int r = (int)(tl % (t.ntx * t.nty * t.ntz));
             const int n = (int)(tl / (t.ntx * t.nty * t.ntz));
             const int oz0 = (r % t.ntz) * 8, oy0 = (r / t.ntz) % t.nty * 16, ox0 = r / (t.ntz * t.nty) * t.TX;
+            // the tile's first voxel inside x: offsets from there
+            const int g0x = max(ox0 * a.s - 1, 0), g0y = max(oy0 * a.s - 1, 0), g0z = max(oz0 * a.s - 1, 0);
             int2* tab = s_tab + b * nvox;
             for (int v = tid; v < nvox; v += kTcWProd) {
                 const int row = v / t.LZ, lx = row / t.LY;
@@ -454,12 +459,12 @@ __global__ void __launch_bounds__(kTcWProd + 32 * kTcIssue, 1) k_conv_tc_wgrad(C
                 const int lz = t.even ? (p < t.even ? 2 * p : 2 * (p - t.even) + 1) : p;
                 const int gx = ox0 * a.s - 1 + lx, gy = oy0 * a.s - 1 + ly, gz = oz0 * a.s - 1 + lz;
                 const bool in = gx >= 0 && gy >= 0 && gz >= 0 && gx < a.X && gy < a.Y && gz < a.Z;
-                tab[v] = make_int2(in ? (gx * a.Y + gy) * a.Z + gz : -1, row * RP + p);
+                tab[v] = make_int2(in ? ((gx - g0x) * a.Y + gy - g0y) * a.Z + gz - g0z : -1, row * RP + p);
             }
             asm volatile("bar.sync 1, %0;" ::"n"(kTcWProd) : "memory");  // the table, among the producers
             if (c >= 2 && !mbar_wait(&s_empty[b], ((c >> 1) - 1) & 1)) ok = false;
             uint8_t* dA = sA + b * a_bytes;
-            const float* x = a.src + (long long)n * a.Cin * Vi;
+            const float* x = a.src + (long long)n * a.Cin * Vi + ((long long)g0x * a.Y + g0y) * a.Z + g0z;
             int h = 0, v = tid;
             while (v >= nvox) v -= nvox, h++;
 #pragma unroll 2
@@ -467,19 +472,19 @@ __global__ void __launch_bounds__(kTcWProd + 32 * kTcIssue, 1) k_conv_tc_wgrad(C
                 const int2 e = tab[v];
                 const int ch0 = ci0 + h * 8, cnt = a.Cin - ch0;
                 *reinterpret_cast<uint4*>(dA + ((size_t)e.y + h * t.LZ) * 16) =
-                    tc_gather8(x + (long long)(cnt > 0 ? ch0 : 0) * Vi + max(e.x, 0), (int)Vi, e.x >= 0, cnt);
+                    tc_gather8(x + (long long)(cnt > 0 ? ch0 : 0) * Vi + max(e.x, 0), Vi, e.x >= 0, cnt);
                 v += kTcWProd;
                 while (v >= nvox) v -= nvox, h++;
             }
             uint8_t* dB = sB + b * b_bytes;
-            const float* dy = a.w + (long long)n * a.Cout * Vo;
+            const float* dy = a.w + (long long)n * a.Cout * Vo + ((long long)ox0 * a.Yo + oy0) * a.Zo + oz0;
             for (int it = tid; it < (t.NT / 8) * nvd; it += kTcWProd) {
                 const int g = it / nvd, q = it - g * nvd;
-                const int ox = ox0 + (q >> 7), oy = oy0 + ((q >> 3) & 15), oz = oz0 + (q & 7);
-                const bool in = ox < a.Xo && oy < a.Yo && oz < a.Zo;
+                const int ox = q >> 7, oy = (q >> 3) & 15, oz = q & 7;
+                const bool in = ox0 + ox < a.Xo && oy0 + oy < a.Yo && oz0 + oz < a.Zo;
                 const int ch0 = co0 + g * 8, cnt = a.Cout - ch0;
                 *reinterpret_cast<uint4*>(dB + (size_t)it * 16) = tc_gather8(
-                    dy + (long long)(cnt > 0 ? ch0 : 0) * Vo + (in ? (ox * a.Yo + oy) * a.Zo + oz : 0), (int)Vo, in, cnt);
+                    dy + (long long)(cnt > 0 ? ch0 : 0) * Vo + (in ? (ox * a.Yo + oy) * a.Zo + oz : 0), Vo, in, cnt);
             }
             fence_async_smem();
             mbar_arrive(&s_full[b]);
@@ -641,6 +646,9 @@ static size_t tc_conv_smem(const ConvTile& t) {
     return t.nbuf * (nvox * 32 + (size_t)27 * 32 * t.NT) + nvox * sizeof(int);
 }
 
+// offsets within a tile of lx planes of an sx x sy x sz grid fit 32 bits
+static bool tc_span(int lx, int sx, int sy, int sz) { return (long long)(lx < sx ? lx : sx) * sy * sz < (1LL << 31); }
+
 template <int MODE>
 static int launch_conv_tc(const ConvTcArgs& a, cudaStream_t st) {
     const int NCH = MODE == 0 ? a.Cout : a.Cin;
@@ -681,7 +689,7 @@ static int launch_conv_tc(const ConvTcArgs& a, cudaStream_t st) {
             c.ntz = (t.QZ + 8 * ZH - 1) / (8 * ZH);
             const long long ctas = (long long)c.ntx * c.nty * c.ntz * a.N * t.nsplit * (half ? 8 : 1);
             const bool two = TX * ZH * t.NT <= 256 && tc_conv_smem(c) <= kTcHalfSmem;
-            const bool fits = TX * ZH * t.NT <= 512 && tc_conv_smem(c) <= kTcMaxSmem;
+            const bool fits = TX * ZH * t.NT <= 512 && tc_conv_smem(c) <= kTcMaxSmem && tc_span(c.LX, t.SX, t.SY, t.SZ);
             const long long score = !fits ? -2 : ctas >= 2 * kNumSM ? (two ? 100 : 0) + TX * ZH * 4 + ZH : 0;
             if (score > best) best = score, pick = c;
         }
@@ -767,7 +775,7 @@ extern "C" int pf_cnn_conv3d_bwd_weight_tc(const float* x, const float* dy, int 
             t.LX = stride * (TX - 1) + 3;
             const size_t vox = (size_t)t.LX * t.LY * t.LZ;
             smem = 2 * (vox * (t.np + 1) * 16 + (size_t)(t.NT / 8) * TX * 128 * 16 + vox * sizeof(int2));
-            found = smem <= kTcMaxSmem;
+            found = smem <= kTcMaxSmem && tc_span(t.LX, X, Y, Z);
         }
     }
     if (!found) return fail(PF_UNSUPPORTED, "tensor-core conv: no tile fits");

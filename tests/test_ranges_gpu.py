@@ -177,6 +177,40 @@ def test_conv_tiles(lib, shape, co, stride):
         assert rel(N(got), N(want)) < 1e-5
 
 
+@pytest.mark.parametrize("stride", [1, 2])
+def test_conv_beyond_32_bit_offsets(lib, stride):
+    # one channel of more than 2^31 voxels, zero but for its last planes: results there as those of a grid that
+    # holds the last planes alone (cut where tiles begin), bitwise for the same products and sums
+    X, Y, Z, tail = 2080, 1024, 1024, 32
+    L, P, s = lib.load(), lib.ptr, lib.stream()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w, b = torch.randn(1, 1, 3, 3, 3, generator=g, device="cuda"), torch.randn(1, generator=g, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    x = torch.zeros(X, Y, Z, device="cuda")
+    x[X - tail + 1:] = torch.randn(tail - 1, Y, Z, generator=g, device="cuda")
+    so = [(v - 1) // stride + 1 for v in (X, Y, Z)]
+    dy = torch.zeros(so, device="cuda")
+    ot = tail // stride  # output planes of the last ones; the first of them stays zero
+    dy[so[0] - ot + 1:] = torch.randn(ot - 1, *so[1:], generator=g, device="cuda")
+
+    def passes(x, dy):
+        n = (1, 1, *x.shape)
+        y, dx, dw, db = torch.empty_like(dy), torch.empty_like(x), torch.empty_like(w), torch.empty_like(b)
+        lib.check(L.pf_cnn_conv3d_fwd_tc(P(x), *n, P(w), P(b), 1, stride, 0, P(y), P(err), s))
+        lib.check(L.pf_cnn_conv3d_bwd_data_tc(P(dy), *n, P(w), 1, stride, 0, P(dx), P(err), s))
+        work = torch.empty(int(L.pf_cnn_conv3d_bwd_weight_tc_workspace(*n, 1, stride)), device="cuda")
+        lib.check(L.pf_cnn_conv3d_bwd_weight_tc(P(x), P(dy), *n, 1, stride, P(dw), P(db), P(work), P(err), s))
+        return y, dx, dw, db
+
+    y, dx, dw, db = passes(x, dy)
+    y1, dx1, dw1, db1 = passes(x[X - tail:].contiguous(), dy[so[0] - ot:].contiguous())
+    assert int(err.item()) == 0
+    assert torch.equal(y[so[0] - ot:], y1) and torch.equal(dx[X - tail:], dx1)
+    assert bool((y[:so[0] - ot - 1] == b).all()) and bool((dx[:X - tail - 1] == 0).all())
+    # the weight gradient's ranges lie elsewhere: sums of up to 33 million products in FP32, by ranges of 4096
+    assert rel(N(dw), N(dw1)) < 1e-4 and rel(N(db), N(db1)) < 1e-4
+
+
 @pytest.mark.parametrize("ext,stride", [((5, 17, 9), 1), ((4, 16, 8), 1), ((3, 5, 3), 1), ((6, 18, 10), 2), ((7, 35, 21), 2),
                                        ((2, 33, 20), 1)])
 @pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
