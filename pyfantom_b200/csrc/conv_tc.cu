@@ -225,9 +225,11 @@ __global__ void __launch_bounds__(kTcProd + 32 * kTcIssue, 2) k_conv_tc(ConvTcAr
     uint8_t* sA = smem;
     uint8_t* sB = smem + t.nbuf * a_bytes;
     int* s_off = reinterpret_cast<int*>(sB + t.nbuf * b_bytes);
-    const int n = blockIdx.y / t.nsplit, j0 = (int)(blockIdx.y % t.nsplit) * t.NT;
+    // tile fastest, then column split, then sample (in one dimension: N * nsplit may exceed 65,535)
+    const unsigned ntile = (unsigned)(t.ntx * t.nty * t.ntz), bt = blockIdx.x % ntile, bs = blockIdx.x / ntile;
+    const int n = (int)(bs / t.nsplit), j0 = (int)(bs % t.nsplit) * t.NT;
     const int par = blockIdx.z, px = par & 1, py = (par >> 1) & 1, pz = par >> 2;  // parity class (stride-2 input gradient)
-    const int bz = blockIdx.x % t.ntz, by = (blockIdx.x / t.ntz) % t.nty, bx = blockIdx.x / (t.ntz * t.nty);
+    const int bz = bt % t.ntz, by = (bt / t.ntz) % t.nty, bx = bt / (t.ntz * t.nty);
     const int q0x = bx * t.TX, q0y = by * 16, q0z = bz * 8 * t.ZH;
     const int nchunk = (KCH + 15) / 16, T = t.TX * t.ZH, nis = min(kTcIssue, T);
     if (warp == 8) {
@@ -698,7 +700,9 @@ static int launch_conv_tc(const ConvTcArgs& a, cudaStream_t st) {
     t.ncols = tc_ncols(t.TX * t.ZH * t.NT);
     const size_t smem = tc_conv_smem(t);
     PF_CUDA(cudaFuncSetAttribute(k_conv_tc<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcMaxSmem));
-    dim3 grid((unsigned)(t.ntx * t.nty * t.ntz), (unsigned)(a.N * t.nsplit), half ? 8u : 1u);
+    const long long blocks = (long long)t.ntx * t.nty * t.ntz * a.N * t.nsplit;
+    if (blocks >= (1LL << 31)) return fail(PF_UNSUPPORTED, "tensor-core conv: %lld tiles", blocks);
+    const dim3 grid((unsigned)blocks, 1, half ? 8u : 1u);
     pf::count_launch();
     k_conv_tc<MODE><<<grid, kTcProd + 32 * kTcIssue, smem, st>>>(a, t);
     PF_LAUNCH_CHECK("tensor-core conv launch");

@@ -177,6 +177,29 @@ def test_conv_tiles(lib, shape, co, stride):
         assert rel(N(got), N(want)) < 1e-5
 
 
+@pytest.mark.parametrize("ci,co,stride", [(1, 240, 1), (200, 2, 1), (130, 1, 2)])
+def test_conv_of_many_samples(lib, ci, co, stride):
+    # samples times column splits beyond 65,535 (three or four splits of the output or input channels)
+    n, ext = 22_000 if max(ci, co) < 150 else 17_000, (2, 1, 1)
+    L, P, s = lib.load(), lib.ptr, lib.stream()
+    g = torch.Generator(device="cuda").manual_seed(9)
+    w, b = torch.randn(co, ci, 3, 3, 3, generator=g, device="cuda").bfloat16().float(), torch.zeros(co, device="cuda")
+    x = torch.randn(n, ci, *ext, generator=g, device="cuda").bfloat16().float()
+    xd, wd = x.double().requires_grad_(), w.double()
+    xp = torch.nn.functional.pad(xd[:, :, :, 0, 0], (1, 1))
+    outs = [torch.einsum("nit,oit->no", xp[:, :, stride * o:stride * o + 3], wd[:, :, :, 1, 1]) for o in range(2 // stride)]
+    ref = torch.stack(outs, 2)[..., None, None]
+    dy = torch.randn(ref.shape, generator=g, device="cuda").bfloat16().float()
+    gx, = torch.autograd.grad(ref, xd, dy.double())
+    y, dx = torch.full_like(dy, np.nan), torch.full_like(x, np.nan)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    lib.check(L.pf_cnn_conv3d_fwd_tc(P(x), n, ci, *ext, P(w), P(b), co, stride, 0, P(y), P(err), s))
+    lib.check(L.pf_cnn_conv3d_bwd_data_tc(P(dy), n, ci, *ext, P(w), co, stride, 0, P(dx), P(err), s))
+    assert int(err.item()) == 0
+    # operands representable in BF16: only the FP32 accumulation differs, as in test_conv_tiles
+    assert rel(N(y), N(ref)) < 1e-5 and rel(N(dx), N(gx)) < 1e-5
+
+
 @pytest.mark.parametrize("stride", [1, 2])
 def test_conv_beyond_32_bit_offsets(lib, stride):
     # one channel of more than 2^31 voxels, zero but for its last planes: results there as those of a grid that
