@@ -452,3 +452,25 @@ def test_vcycle_bottom(nel, nl, ns, kw, precision):
     zr = O.mg_vcycle(nel, unit_K0(3), wl["E"], wl["fixed_dofs"], r, n_level=nl, n_smooth=ns, omega=0.45)
     # FP64: 2 ns products per level of conditioning below 1e5; FP32 carries 1e-7 per operation
     assert rel(z, zr) < (1e-10 if precision == "fp64" else 1e-4)
+
+
+@pytest.mark.parametrize("nel,nl", [((16, 8, 8), 2), ((24, 12, 12), 2), ((48, 24, 24), 3), ((40, 24, 28), 3)])
+@pytest.mark.parametrize("cut", [0.3, 0.6])
+def test_vcycle_bottom_at_solid_and_void(nel, nl, cut):
+    # solid 1 and void 1e-9 element by element, residuals of the size that each node's stiffness gives them.  The
+    # coarsest operator is conditioned below 1e7 by its shift of 1e-6, the rest row by row: 1e-8
+    from test_solver_gpu import setup_problem
+    from conftest import unit_K0
+    from pyfantom_b200 import workloads
+    wl = workloads.cantilever3d(*nel)
+    rng = np.random.default_rng(sum(nel))
+    E = np.where(rng.uniform(size=O.n_elem(nel)) < cut, 1e-9, 1.0)
+    mesh, kern, sol, fe = setup_problem(wl, nl)
+    kern.set_rho(T(E))
+    sol.setup()
+    K0, fixed = unit_K0(3), wl["fixed_dofs"]
+    u = rng.standard_normal(kern.shape[0])
+    r = O.matvec(nel, K0, E, u, fixed)
+    r[fixed] = 0.0
+    z = N(sol.vcycle(T(r), omega=0.45))
+    assert rel(z, O.mg_vcycle(nel, K0, E, fixed, r, n_level=nl, omega=0.45)) < 1e-8
