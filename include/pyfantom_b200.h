@@ -39,7 +39,7 @@ enum pf_status {
     PF_NO_MEMORY = 7,     /* device allocation failed */
     PF_UNSUPPORTED = 8,   /* valid input the library does not handle (e.g. K0 without
                              axis-reflection symmetry) */
-    PF_FACTOR_FAILED = 9  /* coarse Cholesky hit a non-positive pivot */
+    PF_FACTOR_FAILED = 9  /* the coarsest or the direct solve's matrix has a non-positive pivot */
 };
 
 typedef struct pf_grid {
@@ -122,7 +122,7 @@ typedef struct pf_mg_config {
     double omega;       /* reference omega (max omega of the adaptive schedule) */
     double min_omega;   /* reference min_omega argument (effective = max(omega/2, min_omega)) */
     double omega_boost; /* omega growth per level (reference uses 1.06) */
-    double coarse_beta; /* diagonal shift of the coarse Cholesky (CHOLMOD beta = 1e-6) */
+    double coarse_beta; /* diagonal shift of the coarsest operator (CHOLMOD beta = 1e-6) */
     int precision;      /* 0 = FP64 V-cycle, 1 = FP32 V-cycle inside FP64 CG,
                            2 = FP32 V-cycle reading BF16 element scales, inside FP64 CG */
     int check_every;    /* host convergence poll interval in iterations (>= 1) */
@@ -173,7 +173,7 @@ int pf_mg_set_deflation(pf_mg* mg, const double* y, void* stream);
  * the V-cycle precision (double for precision 0, float otherwise).  Requires pf_mg_setup. */
 int pf_mg_level_matvec(pf_mg* mg, int level, const void* u, void* y, void* stream);
 /* h_elem_level1 = 1 if level 1 is applied element by element; h_dirty = its number of
- * coarse elements with an explicit matrix (those touching a constraint). */
+ * coarse elements that touch a constraint (their corners take assembled rows). */
 int pf_mg_level_info(const pf_mg* mg, int* h_elem_level1, int* h_dirty);
 /* Diagnostics: time every fine-level matvec launch of the following solves with CUDA
  * events (at most max_launches per solve; 0 disables), and read the last solve's totals:
@@ -323,8 +323,10 @@ int pf_cnn_energy_loss_f64(long long n, const double* y, const double* Ky, const
 
 /* ---- direct solve for small problems (the reference's SPSOLVE,
  * solvers/CUDA/_solvers.py:245-328 with StructuredStiffnessKernel.construct,
- * stiffness/CUDA/_FEA.py:484-516): dense assembly of the free-DOF block of K(E), tiled
- * Cholesky and inverse factor, x = L^-T L^-1 b; constrained entries of x are b's.
+ * stiffness/CUDA/_FEA.py:484-516).  Half bandwidths of at most 96 (2D grids up to 45
+ * elements across): banded Cholesky from both ends and one correction with the residual in
+ * pairs of doubles.  Others: dense assembly of the free-DOF block of K(E), tiled Cholesky and
+ * inverse factor, x = L^-T L^-1 b.  Constrained entries of x are b's; x may be b.
  * free_dofs [n_free] and dof_to_free [dof] (-1 when constrained) are int32 device
  * arrays; n_free <= 20480. */
 typedef struct pf_direct pf_direct;

@@ -124,9 +124,10 @@ __device__ __forceinline__ void filter_column(const double* s, int plane, const 
 }
 
 // Block: 256 threads, TK columns along z by 256 / TK along y, RI elements along x each.
-// With 27 taps an output costs 9 (RI + 2) / RI shared-memory reads and 27 FMAs.  Bound by
-// instruction issue (2.4 warp instructions per cycle and SM, 24 % of the FP64 pipe), not by
-// its 16 B of DRAM traffic per element.  256x128x128, rmin 2, forward and adjoint together:
+// With 27 taps an output costs 9 (RI + 2) / RI shared-memory reads and 27 FMAs.  No unit is at its
+// limit (ncu, 256x128x128, rmin 2: issue 61 to 63 % of the cycles, shared memory 41 %, FP64 pipe 22 %,
+// DRAM 12 %); the warps, 34 to 40 per SM, mostly wait for the loads that stage the tile, which nothing
+// but other blocks' arithmetic covers.  256x128x128, rmin 2, forward and adjoint together:
 // 76.4 us against 367 us for k_filter; 96x48x48: 14.2 against 29.7 us.  Staging by division-free
 // rows rather than by a flat index took 108 to 97 us, the constant normaliser in the weights 97 to
 // 90 us, the tap table in the kernel's parameters (uniform loads instead of shared-memory ones)

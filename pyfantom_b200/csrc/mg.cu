@@ -1213,7 +1213,7 @@ extern "C" int pf_mg_solve(pf_mg* mg, const double* b, double* x, int use_x0, do
     PF_CUDA(cudaMemcpy(&fpiv, mg->dense.fail, sizeof(int), cudaMemcpyDeviceToHost));
     if (fpiv) {
         if (info) info->status = PF_FACTOR_FAILED;
-        return fail(PF_FACTOR_FAILED, "coarse Cholesky: non-positive pivot at row %d", fpiv - 1);
+        return fail(PF_FACTOR_FAILED, "coarsest operator: non-positive pivot at row %d", fpiv - 1);
     }
     return PF_OK;
 }

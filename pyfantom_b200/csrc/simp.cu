@@ -31,8 +31,8 @@ __device__ __forceinline__ void heavy(double r, double beta, double eta, double*
     *dh = beta * (1.0 - t * t) / den;
 }
 
-// r^e: pow, but for the exponents 0 .. 3 of a penalty of 1 to 4 and its derivative, products (at
-// most two roundings, within pow's own error; pow costs some hundred instructions)
+// r^e: pow, but for the exponents 0 .. 3 of a penalty of 1, 2 or 3 and its derivative, products
+// (at most two roundings, within pow's own error; pow costs some hundred instructions)
 template <int EXP>
 __device__ __forceinline__ double simp_pow(double r, double e) {
     if (EXP == 0) return 1.0;
@@ -339,13 +339,15 @@ __global__ void __launch_bounds__(kRT) k_oc_init_multi(const double* partials, i
 // pass or two of the tree almost every element does.  Where dg is not a finite number >= 0,
 // or ocP vanishes everywhere (x_new = 1e-3 / lambda), every pass covers four levels from the
 // start: more passes, the same sequence.
-// Bound by the FP64 pipe in the first three passes (a product, two comparisons and an FMA
-// per element and midpoint; the reciprocal of the midpoint replaces the division in these
-// sums, x_new itself is divided) and by reading x, ocP and dg (24 B per element, from L2 up
-// to about 4 M elements) in the others.
+// In the sums the reciprocal of the midpoint replaces the division (x_new itself is divided): two
+// roundings per term instead of one, but x_new, lambda and the steps of 100 runs over 16 to 126
+// elements across are bitwise those of the division.
+// No unit is at its limit (ncu, 192x96x96): the first two passes issue in 53 % of the cycles with 16
+// warps per SM (ALU pipe 41 and 48 %: the selects of the two comparisons; FP64 pipe 37 and 34 %; DRAM
+// 19 %), the next two wait for x, ocP and dg (24 B per element, from L2 up to about 4 M elements), the
+// list passes are a chain of latencies (issue 19 %, 12 us cold).  1720 -> 168 us.
 constexpr int kOcStride = 11;
 constexpr int kOcMid = 15;  // midpoints of four bisection levels
-
 
 struct OcSpine {
     int n;

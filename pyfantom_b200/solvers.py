@@ -2,8 +2,8 @@
 
 * ``CG``        - matrix-free unpreconditioned CG (reference :22-132), ``pf_cg_solve``.
 * ``SPSOLVE``   - direct solve for small problems (reference :245-328): the free-DOF block
-  of K assembled dense on the device and factored by the library's tiled Cholesky
-  (``pf_direct_solve_f64``, up to 20,480 free DOFs).
+  of K factored on the device, as a band where it is narrow (2D grids up to 45 elements
+  across), else dense (``pf_direct_solve_f64``, up to 20,480 free DOFs).
 * ``MultiGrid`` - geometric-multigrid-preconditioned CG (reference :330-660) with the
   reference's V-cycle (and its lower-case ``cycle='w'`` W-cycle, which repeats the coarse
   correction at the levels in ``w_level``; the default ``'W'`` runs V-cycles there too),
@@ -108,7 +108,7 @@ class CG(Solver):
 
 class SPSOLVE(Solver):
     """Direct solver (reference _solvers.py:245-328): solves the free DOFs of K(rho) exactly
-    (dense Cholesky on the device) and keeps the right-hand side on constrained DOFs."""
+    (banded or dense Cholesky on the device) and keeps the right-hand side on constrained DOFs."""
 
     def __init__(self, kernel):
         super().__init__()
@@ -263,8 +263,8 @@ class MultiGrid(Solver):
         return y
 
     def level_info(self):
-        """(level 1 applied element by element, number of its coarse elements with an
-        explicit matrix) of the current hierarchy."""
+        """(level 1 applied element by element, number of its coarse elements that touch a
+        constraint) of the current hierarchy."""
         a, b = ctypes.c_int(), ctypes.c_int()
         _lib.check(_lib.load().pf_mg_level_info(self._mg, ctypes.byref(a), ctypes.byref(b)))
         return bool(a.value), int(b.value)
